@@ -30,12 +30,11 @@
 // left out of every restriction and prolongation.
 //
 // Per inner iteration: ml_update (r -= alpha q, T^-1 r, Z_1^T r, r.r and
-// r.T^-1 r in one pass over the node columns), then per coarse level a
-// pre-smoothing (one thread per column) and a residual-with-restriction
-// kernel (one thread per node), the dense coarse product, per level the
-// prolongation and the residual (per node) and a post-smoothing kernel (per
-// column; the top one finishes r.z and beta), and ml_direction (p = T^-1 r + Z_1 c + beta p,
-// x += alpha p).
+// r.T^-1 r in one pass over the node columns, and level 1's pre-smoothing),
+// per coarse level ml_down (the residual, its restriction and the next
+// level's pre-smoothing), the dense coarse product, per level ml_up (the
+// prolonged residual and the post-smoothing; the top one finishes r.z and
+// beta), and ml_direction (p = T^-1 r + Z_1 c + beta p, x += alpha p).
 #pragma once
 
 #include <cuda.h>  // CUtensorMap (the type only; maps are encoded by the host)
@@ -144,6 +143,75 @@ __device__ __forceinline__ bool ml_finish(Acc32 (&acc)[NA], Acc32* scratch, doub
     return threadIdx.x == 0;
 }
 
+// z-line solve of one column held in shared memory: f holds the right-hand
+// side (plane stride `fs`) and receives T^-1 f; l and ip are the column's
+// factors (plane stride `ls`).  The column is read into registers first: the
+// two sweeps are a dependent chain, and one shared-memory round trip per plane
+// would triple it.
+template <int NP>
+__device__ __forceinline__ void ml_sweep_shared(float* f, const float* l, const float* ip, const int L, const int fs,
+                                                const int ls) {
+    float H[NP], Lz[NP], Ip[NP];
+#pragma unroll
+    for (int z = 0; z < NP; ++z) {
+        const int c = z < L ? z : L - 1;
+        H[z] = f[c * fs];
+        Lz[z] = l[c * ls];
+        Ip[z] = ip[c * ls];
+    }
+    float gp = 0.f;
+#pragma unroll
+    for (int z = 0; z < NP; ++z)
+        if (z < L) {
+            gp = fmaf(-Lz[z], gp, H[z]);
+            H[z] = gp * fabsf(Ip[z]);
+        }
+    float wn = 0.f;
+#pragma unroll
+    for (int z = NP - 1; z >= 0; --z)
+        if (z < L) {
+            const float lup = (z + 1 < L) ? Lz[z + 1 < NP ? z + 1 : z] : 0.f;
+            wn = fmaf(-lup, wn, H[z]);
+            f[z * fs] = wn;
+        }
+}
+
+// Pre-smoothing of level 1 (x1 = omega T_1^-1 R_1) by the block that summed
+// R_1: a block of the fine pass owns 2 x 8 level-1 columns with all their
+// planes, so on small boards the sweeps need no kernel of their own (see
+// kMlWidePre).
+// `MLPre` keeps their right-hand sides and z-line factors ([plane][16],
+// column 8 row + column); fetch loads the factors, which no kernel of the
+// iteration writes, ahead of the dependency wait.
+struct MLNext {  // level 1 for its pre-smoothing: z-line factors and iterate (x null: no z-line level)
+    const float *lf, *ipd;
+    float* x;
+};
+template <int NP>
+struct MLPre {
+    float r[NP][16], lf[NP][16], ip[NP][16];
+    __device__ __forceinline__ void fetch(const MLNext& nx, const MLGrid& g1, int by, int bx) {
+        for (int k = threadIdx.x; k < 16 * g1.L; k += blockDim.x) {
+            const int AY = by * 2 + ((k >> 3) & 1), AX = bx * 8 + (k & 7);
+            const bool in = AY < g1.ny && AX < g1.nx;
+            const long long i = in ? ml_index(g1, k >> 4, AY, AX) : 0;
+            lf[k >> 4][k & 15] = in ? __ldg(nx.lf + i) : 0.f;
+            ip[k >> 4][k & 15] = in ? __ldg(nx.ipd + i) : 0.f;
+        }
+    }
+    // every thread of the block, r complete except for a barrier
+    __device__ __forceinline__ void smooth(const MLNext& nx, const MLGrid& g1, int by, int bx) {
+        __syncthreads();
+        if (threadIdx.x < 16)
+            ml_sweep_shared<NP>(&r[0][threadIdx.x], &lf[0][threadIdx.x], &ip[0][threadIdx.x], g1.L, 16, 16);
+        __syncthreads();
+        for (int k = threadIdx.x; k < 16 * g1.L; k += blockDim.x) {
+            const int AY = by * 2 + ((k >> 3) & 1), AX = bx * 8 + (k & 7);
+            if (AY < g1.ny && AX < g1.nx) nx.x[ml_index(g1, k >> 4, AY, AX)] = kMlOmega * r[k >> 4][k & 15];
+        }
+    }
+};
+
 // ------------------------------------------------------------ fine level
 // One pass over the fine node columns.  Thread (lane, warp) of block (bx, by)
 // owns node column x = 32 bx + lane of node row y = 8 by + warp and walks the
@@ -162,11 +230,13 @@ template <int NP, int MODE>
 __global__ void __launch_bounds__(kMlThreads)
     ml_update(float* __restrict__ r, const float* __restrict__ q, const double* __restrict__ r64,
               float* __restrict__ x32, float* __restrict__ w, float* __restrict__ R1, const float* __restrict__ zl,
-              const float* __restrict__ zi, Layout lay, long long pstride, MLGrid g1, SolveCtl* ctl,
+              const float* __restrict__ zi, Layout lay, long long pstride, MLGrid g1, MLNext nx, SolveCtl* ctl,
               double* partials, unsigned int* counter, KernelClock* clock) {
     __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc32) * 2 * 32];
     __shared__ float s_part[NP][8][8];  // [plane][row of the block][aggregate column of the block]
+    __shared__ MLPre<NP> s_pre;
     Acc32* const scratch = reinterpret_cast<Acc32*>(scratch_raw);
+    if (nx.x != nullptr) s_pre.fetch(nx, g1, blockIdx.y, blockIdx.x);
     pdl_enter();
     if ((MODE == ML_ITER || MODE == ML_PRE64) && ctl->state != ST_RUNNING) return;
     if (MODE == ML_ITER && clock != nullptr && threadIdx.x == 0) atomicMin(&clock->first, global_ns());
@@ -240,12 +310,13 @@ __global__ void __launch_bounds__(kMlThreads)
     for (int k = threadIdx.x; k < 16 * np; k += blockDim.x) {
         const int z = k >> 4, a_row = (k >> 3) & 1, a_col = k & 7;
         const int AY = blockIdx.y * 2 + a_row, AX = blockIdx.x * 8 + a_col;
-        if (AY < g1.ny && AX < g1.nx) {
-            const float(&b)[8][8] = s_part[z];
-            const int w0 = 4 * a_row;
-            R1[ml_index(g1, z, AY, AX)] = (b[w0][a_col] + b[w0 + 1][a_col]) + (b[w0 + 2][a_col] + b[w0 + 3][a_col]);
-        }
+        const float(&b)[8][8] = s_part[z];
+        const int w0 = 4 * a_row;
+        const float sum = (b[w0][a_col] + b[w0 + 1][a_col]) + (b[w0 + 2][a_col] + b[w0 + 3][a_col]);
+        if (AY < g1.ny && AX < g1.nx) R1[ml_index(g1, z, AY, AX)] = sum;
+        s_pre.r[z][k & 15] = sum;
     }
+    if (nx.x != nullptr) s_pre.smooth(nx, g1, blockIdx.y, blockIdx.x);
     if (MODE == ML_ONLY) return;
     Acc32 acc[2], tot[2];
     acc[0].s = rr;
@@ -288,11 +359,12 @@ struct MLStageMaps {
 template <int NP>
 __global__ void __launch_bounds__(kMlThreads, 1)
     ml_update_staged(float* __restrict__ r, float* __restrict__ w, float* __restrict__ R1, Layout lay,
-                     long long pstride, MLGrid g1, SolveCtl* ctl, double* partials, unsigned int* counter,
+                     long long pstride, MLGrid g1, MLNext nx, SolveCtl* ctl, double* partials, unsigned int* counter,
                      KernelClock* clock, int tiles_x, int tiles, int stages, const __grid_constant__ MLStageMaps M) {
     extern __shared__ __align__(128) unsigned char ml_stage_raw[];
     __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc32) * 2 * 32];
     __shared__ float s_part[NP][8][8];  // [plane][row of the tile][aggregate column of the tile]
+    __shared__ MLPre<NP> s_pre;
     __shared__ __align__(8) unsigned long long s_bar[kMlMaxStages];
     Acc32* const scratch = reinterpret_cast<Acc32*>(scratch_raw);
     // tensor copies write 128-byte aligned boxes: the launch adds 128 bytes
@@ -397,13 +469,17 @@ __global__ void __launch_bounds__(kMlThreads, 1)
         for (int i = tid; i < 16 * np; i += blockDim.x) {
             const int z = i >> 4, a_row = (i >> 3) & 1, a_col = i & 7;
             const int AY = ty * 2 + a_row, AX = tx * 8 + a_col;
-            if (AY < g1.ny && AX < g1.nx) {
-                const float(&b)[8][8] = s_part[z];
-                const int w0 = 4 * a_row;
-                R1[ml_index(g1, z, AY, AX)] = (b[w0][a_col] + b[w0 + 1][a_col]) + (b[w0 + 2][a_col] + b[w0 + 3][a_col]);
-            }
+            const float(&b)[8][8] = s_part[z];
+            const int w0 = 4 * a_row;
+            const float sum = (b[w0][a_col] + b[w0 + 1][a_col]) + (b[w0 + 2][a_col] + b[w0 + 3][a_col]);
+            if (AY < g1.ny && AX < g1.nx) R1[ml_index(g1, z, AY, AX)] = sum;
+            s_pre.r[z][i & 15] = sum;
         }
-        // the next tile's s_part writes follow its stage vote, a barrier
+        if (nx.x != nullptr) {
+            s_pre.fetch(nx, g1, ty, tx);
+            s_pre.smooth(nx, g1, ty, tx);
+        }
+        // the next tile's s_part and s_pre writes follow its stage vote, a barrier
     }
     Acc32 tot[2];
     if (ml_finish<2>(acc, scratch, partials, counter, tot)) {
@@ -560,228 +636,512 @@ __global__ void __launch_bounds__(kVecThreads)
 }
 
 // ------------------------------------------------------------ coarse levels
-// Two thread layouts: the z-line kernels give each thread one node column
-// (all planes, a 1D grid over the columns); the residual kernels give each
-// thread one node (block = 32 columns x 8 rows of one plane, grid.z = plane),
-// so the 27-point stencils of a level run fully in parallel.
+// Two kernels per level.  A block owns 16 x 4 node columns with all their
+// planes; its 64 ml_level_groups(L) threads take one column each of the group's
+// planes (z = group, group + groups, ...), so that a small grid still has a
+// node per thread and a block can run the z-line sweeps of its columns itself.
+//
+//   ml_down: s = R - A x (x the pre-smoothed iterate from zero), its
+//     aggregate sums Rc, and with a z-line level below that level's own
+//     pre-smoothing xc = omega Tc^-1 Rc, whose columns lie in the block.
+//   ml_up: t = s - (A Z) c, y = x + Z c + omega T^-1 t.  A Z couples a node
+//     with at most 2 x 2 aggregates of three planes: 12 coefficients built at
+//     set-up take the place of the 27-point stencil on x + Z c.
+//
+// What bounds them and what the split measured (B200): a large level (c3's
+// first, 17 x 513 x 513) streams its coefficients (down 76 bytes a node, up
+// 72); a small one is a chain of kernel boundaries and L2 round trips, so the
+// constant coefficients are loaded before the dependency wait where a thread
+// has at most kMlPreRounds nodes.  Five kernels per level (pre-smoothing,
+// restriction, prolongation, residual, post-smoothing) became two: an iteration
+// takes 30.9 us instead of 40.8 on a 71 x 93 x 8 board, 96.4 instead of 118.5
+// on c2 (512 x 512 x 12).
+constexpr int kMlColX = 16, kMlColY = 4;  // node columns of a block
+constexpr int kMlCols = kMlColX * kMlColY;
+constexpr int kMlMaxGroups = 9;           // plane groups of a block: 576 threads at most
+constexpr int kMlPreRounds = 2;           // nodes per thread whose coefficients are loaded ahead of the wait
+constexpr int kMlAz = 12;                 // coefficients of A Z per node: plane (3) x row {own, side} x column {own, side}
 
-// x = omega T^-1 R on column c of level g (pre-smoothing from zero): every
-// plane's loads first, at clamped addresses, then the sweeps.
-template <int NP>
-__device__ __forceinline__ void ml_presmooth_column(const float* __restrict__ R, float* __restrict__ xo,
-                                                    const float* __restrict__ lf, const float* __restrict__ ipd,
-                                                    const MLGrid& g, long long c) {
-    float H[NP], Lz[NP], Ip[NP];
+__host__ __device__ constexpr int ml_level_rounds(int L) { return (L + kMlMaxGroups - 1) / kMlMaxGroups; }
+__host__ __device__ constexpr int ml_level_groups(int L) { return (L + ml_level_rounds(L) - 1) / ml_level_rounds(L); }
+
+// The 27 coefficients of node (z, y, x) in the order of ml_stencil_dot, zero
+// outside the grid.
+__device__ __forceinline__ void ml_load_stencil(float (&a)[27], const float* __restrict__ st, const MLGrid& g, int z,
+                                                int y, int x) {
+    const int n = (int)g.n, plane = (int)g.plane, nx = g.nx;
+    const int i = z * plane + y * nx + x;
+#pragma unroll
+    for (int o = 0; o < 27; ++o) {
+        const int dz = o / 9 - 1, dy = (o / 3) % 3 - 1, dx = o % 3 - 1;
+        const bool in = z + dz >= 0 && z + dz < g.L && y + dy >= 0 && y + dy < g.ny && x + dx >= 0 && x + dx < nx;
+        const int j = i + dz * plane + dy * nx + dx;
+        a[o] = in ? __ldg(o >= 13 ? st + (o - 13) * n + i : st + (13 - o) * n + j) : 0.f;
+    }
+}
+__device__ __forceinline__ float ml_stencil_dot_held(const float (&a)[27], const float* __restrict__ v,
+                                                     const MLGrid& g, int z, int y, int x) {
+    float acc = 0.f;
+#pragma unroll
+    for (int o = 0; o < 27; ++o) {
+        // outside the grid the coefficient is zero: any valid address serves
+        const int jz = min(max(z + o / 9 - 1, 0), g.L - 1), jy = min(max(y + (o / 3) % 3 - 1, 0), g.ny - 1);
+        const int jx = min(max(x + o % 3 - 1, 0), g.nx - 1);
+        acc = fmaf(a[o], v[jz * (int)g.plane + jy * g.nx + jx], acc);
+    }
+    return acc;
+}
+
+// Shared memory of ml_down and ml_up (floats): the block's node values, and
+// the z-line factors of the columns the block sweeps.
+inline size_t ml_level_smem(int L) { return (size_t)3 * L * kMlCols * sizeof(float); }
+
+// PRE: a thread holds the coefficients of its ml_level_rounds(L) <=
+// kMlPreRounds nodes, loaded before the wait (grids of at most a few blocks
+// per SM, where the wait is the larger part of the kernel).
+template <int B, int ROUNDS, bool PRE>
+__global__ void __launch_bounds__(kMlCols* kMlMaxGroups)
+    ml_down(const float* __restrict__ st, const float* R, const float* xv, const float* __restrict__ ipd, float* sv,
+            float* Rc, float* xc, const float* __restrict__ lfc, const float* __restrict__ ipdc, MLGrid g, MLGrid gc,
+            const SolveCtl* ctl) {
+    static_assert(B == 2 || B == 4, "aggregates are 2 x 2 or 4 x 4 node columns");
+    constexpr int CX = kMlColX / B, CY = kMlColY / B, CC = CX * CY;  // coarse columns of the block
+    extern __shared__ float ml_sm[];
+    float* const s_val = ml_sm;                  // [L][kMlCols] residuals, then [L][CC] coarse right-hand sides
+    float* const s_lf = ml_sm + g.L * kMlCols;   // [L][CC] factors of the coarse columns
+    float* const s_ip = s_lf + g.L * CC;
+    const int t = threadIdx.x, col = t & (kMlCols - 1), grp = t / kMlCols, groups = blockDim.x / kMlCols;
+    const int x = blockIdx.x * kMlColX + (col & (kMlColX - 1)), y = blockIdx.y * kMlColY + col / kMlColX;
+    const bool mine = x < g.nx && y < g.ny;
+    float a[PRE ? ROUNDS : 1][27], ip[PRE ? ROUNDS : 1];
+    if (PRE) {
+#pragma unroll
+        for (int k = 0; k < ROUNDS; ++k) {
+            const int z = grp + k * groups;
+            if (mine && z < g.L) {
+                ml_load_stencil(a[k], st, g, z, y, x);
+                ip[k] = __ldg(ipd + ml_index(g, z, y, x));
+            } else {
+#pragma unroll
+                for (int o = 0; o < 27; ++o) a[k][o] = 0.f;
+                ip[k] = -1.f;
+            }
+        }
+    }
+    if (xc != nullptr && t < g.L * CC) {
+        const int z = t / CC, c = t % CC;
+        const int AX = blockIdx.x * CX + c % CX, AY = blockIdx.y * CY + c / CX;
+        const bool in = AX < gc.nx && AY < gc.ny;
+        s_lf[t] = in ? __ldg(lfc + ml_index(gc, z, AY, AX)) : 0.f;
+        s_ip[t] = in ? __ldg(ipdc + ml_index(gc, z, AY, AX)) : 0.f;
+    }
+    pdl_enter();
+    if (ctl != nullptr && ctl->state != ST_RUNNING) return;
+    if (PRE) {
+#pragma unroll
+        for (int k = 0; k < ROUNDS; ++k) {
+            const int z = grp + k * groups;
+            if (z < g.L) {
+                float v = 0.f;
+                if (mine) {
+                    const int idx = (int)ml_index(g, z, y, x);
+                    v = R[idx] - ml_stencil_dot_held(a[k], xv, g, z, y, x);
+                    sv[idx] = v;
+                    if (!(ip[k] >= 0.f)) v = 0.f;
+                }
+                s_val[z * kMlCols + col] = v;
+            }
+        }
+    } else {
+        for (int z = grp; z < g.L; z += groups) {
+            float v = 0.f;
+            if (mine) {
+                const int idx = (int)ml_index(g, z, y, x);
+                v = R[idx] - (ml_interior(g, z, y, x) ? ml_stencil_dot<true>(st, xv, g, z, y, x)
+                                                      : ml_stencil_dot<false>(st, xv, g, z, y, x));
+                sv[idx] = v;
+                if (!(ipd[idx] >= 0.f)) v = 0.f;
+            }
+            s_val[z * kMlCols + col] = v;
+        }
+    }
+    __syncthreads();
+    // aggregate sums: coarse column c of plane z, rows in order, pairs along x first
+    // (L CC <= blockDim: one per thread)
+    float sum = 0.f;
+    if (t < g.L * CC) {
+        const int z = t / CC, c = t % CC;
+        const float* const v = s_val + z * kMlCols + (c / CX) * B * kMlColX + (c % CX) * B;
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const float* const w = v + u * kMlColX;
+            sum += (B == 4) ? (w[0] + w[1]) + (w[2] + w[3]) : w[0] + w[1];
+        }
+        const int AX = blockIdx.x * CX + c % CX, AY = blockIdx.y * CY + c / CX;
+        if (AX < gc.nx && AY < gc.ny) Rc[ml_index(gc, z, AY, AX)] = sum;
+    }
+    if (xc == nullptr) return;
+    __syncthreads();  // the residuals are summed: their place takes the coarse right-hand sides
+    if (t < g.L * CC) s_val[t] = sum;
+    __syncthreads();
+    if (t < CC) ml_sweep_shared<ROUNDS * kMlMaxGroups>(s_val + t, s_lf + t, s_ip + t, g.L, CC, CC);
+    __syncthreads();
+    if (t < g.L * CC) {
+        const int z = t / CC, c = t % CC;
+        const int AX = blockIdx.x * CX + c % CX, AY = blockIdx.y * CY + c / CX;
+        if (AX < gc.nx && AY < gc.ny) xc[ml_index(gc, z, AY, AX)] = kMlOmega * s_val[t];
+    }
+}
+
+// (A Z c) at a node: own aggregate (Y, X) of plane z, the aggregates beside it
+// (dY, dX: -1 or +1) and the planes below and above.  Aggregates and planes
+// outside the grid have zero coefficients; their addresses are clamped.
+template <bool HELD>
+__device__ __forceinline__ float ml_az_dot(const float (&a)[kMlAz], const float* __restrict__ az, const float* cn,
+                                           const MLGrid& g, const MLGrid& gc, int idx, int z, int Y, int X, int dY,
+                                           int dX) {
+    const int Ys = min(max(Y + dY, 0), gc.ny - 1), Xs = min(max(X + dX, 0), gc.nx - 1);
+    float acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < kMlAz; ++k) {
+        const int jz = min(max(z + k / 4 - 1, 0), g.L - 1);
+        const int j = jz * (int)gc.plane + ((k & 2) ? Ys : Y) * gc.nx + ((k & 1) ? Xs : X);
+        acc = fmaf(HELD ? a[k] : __ldg(az + k * (int)g.n + idx), cn[j], acc);
+    }
+    return acc;
+}
+
+// r.z = r.T^-1 r + R.y of the top coarse level, and for an iteration beta and
+// the iteration limit.
+__device__ __forceinline__ void ml_finish_rz(SolveCtl* ctl, double ry, int mode) {
+    const double rzn = ctl->rdr + ry;
+    if (mode == ML_START) {
+        ctl->rz = rzn;
+    } else if (!isfinite(rzn) || ctl->rz == 0.0) {
+        ctl->state = ST_BREAKDOWN;
+    } else {
+        ctl->beta = rzn / ctl->rz;
+        ctl->rz = rzn;
+        if (ctl->iterations >= ctl->max_it) ctl->state = ST_MAXIT;
+    }
+}
+
+// TOP: the first coarse level, where the last block also finishes r.z = r.T^-1 r
+// + R.y and, for ML_ITER, beta and the iteration limit; ML_START sets r.z.
+// ROUNDS: nodes per thread, ml_level_rounds(L).
+template <int B, int ROUNDS, bool TOP>
+__global__ void __launch_bounds__(kMlCols* kMlMaxGroups)
+    ml_up(const float* __restrict__ az, const float* R, const float* sv, const float* xv, const float* cn,
+          const float* __restrict__ lf, const float* __restrict__ ipd, float* yo, MLGrid g, MLGrid gc, SolveCtl* ctl,
+          int mode, double* partials, unsigned int* counter) {
+    constexpr bool PRE = ROUNDS <= kMlPreRounds;
+    __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc32) * 32];
+    Acc32* const scratch = reinterpret_cast<Acc32*>(scratch_raw);
+    extern __shared__ float ml_sm[];
+    float* const s_t = ml_sm;                   // [L][kMlCols]
+    float* const s_lf = s_t + g.L * kMlCols;    // [L][kMlCols]
+    float* const s_ip = s_lf + g.L * kMlCols;   // [L][kMlCols]
+    const int t = threadIdx.x, col = t & (kMlCols - 1), grp = t / kMlCols, groups = blockDim.x / kMlCols;
+    const int x = blockIdx.x * kMlColX + (col & (kMlColX - 1)), y = blockIdx.y * kMlColY + col / kMlColX;
+    const bool mine = x < g.nx && y < g.ny;
+    const int xl = mine ? x : 0, yl = mine ? y : 0;  // clamped: valid addresses, results unused
+    const int Y = yl / B, X = xl / B;
+    const int dY = (yl - Y * B < B / 2) ? -1 : 1, dX = (xl - X * B < B / 2) ? -1 : 1;
+    float a[PRE ? ROUNDS : 1][kMlAz];
+    bool live[ROUNDS];
+#pragma unroll
+    for (int k = 0; k < ROUNDS; ++k) {
+        const int z = grp + k * groups;
+        const bool in = z < g.L;
+        const int idx = (int)ml_index(g, in ? z : 0, yl, xl);
+        const float p = __ldg(ipd + idx);
+        live[k] = p >= 0.f;
+        if (PRE) {
+#pragma unroll
+            for (int m = 0; m < kMlAz; ++m) a[PRE ? k : 0][m] = __ldg(az + m * (int)g.n + idx);
+        }
+        if (in) {
+            s_lf[z * kMlCols + col] = __ldg(lf + idx);
+            s_ip[z * kMlCols + col] = p;
+        }
+    }
+    pdl_enter();
+    if (mode != ML_ONLY && ctl->state != ST_RUNNING) return;
+    float yp[ROUNDS], rv[ROUNDS];
+#pragma unroll
+    for (int k = 0; k < ROUNDS; ++k) {
+        const int z = grp + k * groups;
+        yp[k] = 0.f;
+        rv[k] = 0.f;
+        if (z < g.L) {
+            const int idx = (int)ml_index(g, z, yl, xl);
+            const float c0 = cn[z * (int)gc.plane + Y * gc.nx + X];
+            yp[k] = xv[idx] + (live[k] ? c0 : 0.f);
+            if (TOP && mode != ML_ONLY) rv[k] = R[idx];
+            s_t[z * kMlCols + col] = sv[idx] - ml_az_dot<PRE>(a[PRE ? k : 0], az, cn, g, gc, idx, z, Y, X, dY, dX);
+        }
+    }
+    __syncthreads();
+    if (t < kMlCols) ml_sweep_shared<ROUNDS * kMlMaxGroups>(s_t + t, s_lf + t, s_ip + t, g.L, kMlCols, kMlCols);
+    __syncthreads();
+    Acc32 acc[1];
+#pragma unroll
+    for (int k = 0; k < ROUNDS; ++k) {
+        const int z = grp + k * groups;
+        if (mine && z < g.L) {
+            const float yv = fmaf(kMlOmega, s_t[z * kMlCols + col], yp[k]);
+            yo[ml_index(g, z, y, x)] = yv;
+            if (TOP && mode != ML_ONLY) acc[0].add_product(rv[k], yv);
+        }
+    }
+    if (!TOP || mode == ML_ONLY) return;
+    Acc32 tot[1];
+    if (ml_finish<1>(acc, scratch, partials, counter, tot)) ml_finish_rz(ctl, tot[0].value(), mode);
+}
+
+// ------------------------------------------------ coarse levels, wide grids
+// The same two steps with one thread per node column, for levels wide enough
+// to fill the device with columns: a thread marches its column bottom to top
+// with the neighbours' values of three planes in registers (9 new values per
+// plane instead of 27 per node; 4 aggregate values instead of 12), so that
+// almost every load is a coefficient, used once, and many of them are in
+// flight without a barrier between.  The next plane's loads are issued before a
+// plane is computed: without that a block spent 4.4 us per plane on a chain of
+// round trips (ml_up_wide 227 us on c3's first level, now 85: 3.8 TB/s of its 72
+// bytes a node; ml_down_wide 120, now 108: 3.1 TB/s).
+constexpr int kMlWideX = 32, kMlWideY = 4;  // columns of a block of ml_down_wide
+constexpr int kMlWideThreads = kMlWideX * kMlWideY;
+
+template <int NP, int B>
+__global__ void __launch_bounds__(kMlWideThreads, 4)
+    ml_down_wide(const float* __restrict__ st, const float* __restrict__ R, const float* __restrict__ xv,
+                 const float* __restrict__ ipd, float* __restrict__ sv, float* __restrict__ Rc, float* xc,
+                 const float* __restrict__ lfc, const float* __restrict__ ipdc, MLGrid g, MLGrid gc,
+                 const SolveCtl* ctl) {
+    constexpr int CX = kMlWideX / B, CY = kMlWideY / B, CC = CX * CY;  // coarse columns of the block
+    __shared__ float s_part[NP][kMlWideY][CX];  // per node row: sums over the row's part of an aggregate
+    __shared__ float s_r[NP][CC], s_lf[NP][CC], s_ip[NP][CC];
+    const int t = threadIdx.x, lane = t & 31, row = t >> 5;
+    const int x = blockIdx.x * kMlWideX + lane, y = blockIdx.y * kMlWideY + row;
+    const bool mine = x < g.nx && y < g.ny;
+    const int n = (int)g.n, plane = (int)g.plane, nx = g.nx;
+    if (xc != nullptr)
+        for (int e = t; e < g.L * CC; e += kMlWideThreads) {
+            const int z = e / CC, c = e % CC;
+            const int AX = blockIdx.x * CX + c % CX, AY = blockIdx.y * CY + c / CX;
+            const bool in = AX < gc.nx && AY < gc.ny;
+            const int i = in ? (int)ml_index(gc, z, AY, AX) : 0;
+            s_lf[z][c] = in ? __ldg(lfc + i) : 0.f;
+            s_ip[z][c] = in ? __ldg(ipdc + i) : 0.f;
+        }
+    // in-plane neighbours k = 3 (dy + 1) + (dx + 1): their offsets in a plane
+    // (clamped), and whether they exist: the value of one that does not is 0,
+    // so that whatever coefficient its clamped address holds drops out
+    int off[9];
+    bool in[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const int jy = y + k / 3 - 1, jx = x + k % 3 - 1;
+        in[k] = mine && jy >= 0 && jy < g.ny && jx >= 0 && jx < nx;
+        off[k] = in[k] ? jy * nx + jx : 0;
+    }
+    pdl_enter();
+    if (ctl != nullptr && ctl->state != ST_RUNNING) return;
+    // The coefficients, R and 1/p of the next plane and the values of the plane
+    // above it are loaded before a plane is computed.
+    float X[4][9];  // the neighbours' values on planes z - 1, z, z + 1 and (in flight) z + 2
+    float A[27], rz, pz;
+    auto fetch = [&](const int z) {  // plane z (clamped) into A, rz, pz
+        const int zc = min(z, g.L - 1), zp = zc * plane, zm = max(zc - 1, 0) * plane, i = zp + off[4];
+#pragma unroll
+        for (int o = 0; o < 27; ++o)
+            A[o] = __ldg(st + (o >= 13 ? (o - 13) * n + i : (13 - o) * n + (o < 9 ? zm + off[o] : zp + off[o - 9])));
+        rz = R[i];
+        pz = ipd[i];
+    };
+    auto values = [&](float (&v)[9], const int z) {
+        const int zc = min(z, g.L - 1) * plane;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) v[k] = (in[k] && z < g.L) ? xv[zc + off[k]] : 0.f;
+    };
+#pragma unroll
+    for (int k = 0; k < 9; ++k) X[0][k] = 0.f;
+    values(X[1], 0);
+    values(X[2], 1);
+    fetch(0);
 #pragma unroll
     for (int z = 0; z < NP; ++z) {
-        const long long idx = (long long)(z < g.L ? z : g.L - 1) * g.plane + c;
+        if (z < g.L) {
+            float a[27];
+#pragma unroll
+            for (int o = 0; o < 27; ++o) a[o] = A[o];
+            const float rc = rz, pc = pz;
+            fetch(z + 1);
+            values(X[3], z + 2);
+            float acc = 0.f;
+#pragma unroll
+            for (int o = 0; o < 27; ++o) acc = fmaf(a[o], X[o / 9][o % 9], acc);
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                X[0][k] = X[1][k];
+                X[1][k] = X[2][k];
+                X[2][k] = X[3][k];
+            }
+            float v = 0.f;
+            if (mine) {
+                v = rc - acc;
+                sv[z * plane + off[4]] = v;
+                if (!(pc >= 0.f)) v = 0.f;
+            }
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            if (B == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
+            if ((lane & (B - 1)) == 0) s_part[z][row][lane / B] = v;
+        }
+    }
+    __syncthreads();
+    for (int e = t; e < g.L * CC; e += kMlWideThreads) {
+        const int z = e / CC, c = e % CC, w0 = (c / CX) * B;
+        float sum = s_part[z][w0][c % CX] + s_part[z][w0 + 1][c % CX];
+        if (B == 4) sum += s_part[z][(w0 + 2) % kMlWideY][c % CX] + s_part[z][(w0 + 3) % kMlWideY][c % CX];
+        const int AX = blockIdx.x * CX + c % CX, AY = blockIdx.y * CY + c / CX;
+        if (AX < gc.nx && AY < gc.ny) Rc[ml_index(gc, z, AY, AX)] = sum;
+        s_r[z][c] = sum;
+    }
+    if (xc == nullptr) return;
+    __syncthreads();
+    if (t < CC) ml_sweep_shared<NP>(&s_r[0][t], &s_lf[0][t], &s_ip[0][t], g.L, CC, CC);
+    __syncthreads();
+    for (int e = t; e < g.L * CC; e += kMlWideThreads) {
+        const int z = e / CC, c = e % CC;
+        const int AX = blockIdx.x * CX + c % CX, AY = blockIdx.y * CY + c / CX;
+        if (AX < gc.nx && AY < gc.ny) xc[ml_index(gc, z, AY, AX)] = kMlOmega * s_r[z][c];
+    }
+}
+
+template <int NP, int B, bool TOP>
+__global__ void __launch_bounds__(kMlWideThreads, NP <= 18 ? 4 : 3)
+    ml_up_wide(const float* __restrict__ az, const float* __restrict__ R, const float* __restrict__ sv,
+               const float* __restrict__ xv, const float* __restrict__ cn, const float* __restrict__ lf,
+               const float* __restrict__ ipd, float* __restrict__ yo, MLGrid g, MLGrid gc, SolveCtl* ctl,
+               int mode, double* partials, unsigned int* counter) {
+    __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc32) * 32];
+    Acc32* const scratch = reinterpret_cast<Acc32*>(scratch_raw);
+    const int n = (int)g.n, plane = (int)g.plane, cplane = (int)gc.plane;
+    const int c = blockIdx.x * kMlWideThreads + threadIdx.x;
+    const bool mine = c < plane;
+    const int cl = mine ? c : plane - 1;  // clamped: valid addresses, results unused
+    const int y = cl / g.nx, x = cl - y * g.nx;
+    const int Y = y / B, X = x / B;
+    const int Ys = min(max(Y + ((y - Y * B < B / 2) ? -1 : 1), 0), gc.ny - 1);
+    const int Xs = min(max(X + ((x - X * B < B / 2) ? -1 : 1), 0), gc.nx - 1);
+    const int co[4] = {Y * gc.nx + X, Y * gc.nx + Xs, Ys * gc.nx + X, Ys * gc.nx + Xs};
+    pdl_enter();
+    if (mode != ML_ONLY && ctl->state != ST_RUNNING) return;
+    // Every load of the next plane is issued before a plane is computed.
+    float C[4][4];  // own and side aggregates on planes z - 1, z, z + 1 (zero coefficients outside) and z + 2
+    float A[kMlAz], sz, xz, lz, pz;
+    auto fetch = [&](const int z) {
+        const int idx = min(z, g.L - 1) * plane + cl;
+#pragma unroll
+        for (int k = 0; k < kMlAz; ++k) A[k] = __ldg(az + k * n + idx);
+        sz = sv[idx];
+        xz = xv[idx];
+        lz = lf[idx];
+        pz = ipd[idx];
+    };
+    auto values = [&](float (&v)[4], const int z) {
+        const int zc = min(z, g.L - 1) * cplane;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = cn[zc + co[k]];
+    };
+#pragma unroll
+    for (int k = 0; k < 4; ++k) C[0][k] = 0.f;
+    values(C[1], 0);
+    values(C[2], 1);
+    fetch(0);
+    float H[NP], Lz[NP], Yp[NP];
+    float gp = 0.f;
+#pragma unroll
+    for (int z = 0; z < NP; ++z) {
+        if (z < g.L) {
+            float a[kMlAz];
+#pragma unroll
+            for (int k = 0; k < kMlAz; ++k) a[k] = A[k];
+            const float s0 = sz, x0 = xz, l0 = lz, p0 = pz;
+            fetch(z + 1);
+            values(C[3], z + 2);
+            float acc = 0.f;
+#pragma unroll
+            for (int k = 0; k < kMlAz; ++k) acc = fmaf(a[k], C[k / 4][k % 4], acc);
+            Yp[z] = x0 + (p0 >= 0.f ? C[1][0] : 0.f);
+            Lz[z] = l0;
+            gp = fmaf(-l0, gp, s0 - acc);
+            H[z] = gp * fabsf(p0);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                C[0][k] = C[1][k];
+                C[1][k] = C[2][k];
+                C[2][k] = C[3][k];
+            }
+        }
+    }
+    float Rv[NP];
+    if (TOP && mode != ML_ONLY) {
+#pragma unroll
+        for (int z = 0; z < NP; ++z) Rv[z] = R[min(z, g.L - 1) * plane + cl];
+    }
+    Acc32 acc[1];
+    float wn = 0.f;
+#pragma unroll
+    for (int z = NP - 1; z >= 0; --z) {
+        if (z < g.L) {
+            const float lup = (z + 1 < g.L) ? Lz[z + 1 < NP ? z + 1 : z] : 0.f;
+            wn = fmaf(-lup, wn, H[z]);
+            const float yv = fmaf(kMlOmega, wn, Yp[z]);
+            if (mine) {
+                yo[z * plane + cl] = yv;
+                if (TOP && mode != ML_ONLY) acc[0].add_product(Rv[z], yv);
+            }
+        }
+    }
+    if (!TOP || mode == ML_ONLY) return;
+    Acc32 tot[1];
+    if (ml_finish<1>(acc, scratch, partials, counter, tot)) ml_finish_rz(ctl, tot[0].value(), mode);
+}
+
+// Pre-smoothing x = omega T^-1 R of level 1 as a kernel of its own, one column
+// per thread (see MLPre).
+template <int NP>
+__global__ void __launch_bounds__(kMlWideThreads)
+    ml_presmooth(const float* __restrict__ R, float* __restrict__ xo, const float* __restrict__ lf,
+                 const float* __restrict__ ipd, MLGrid g, const SolveCtl* ctl) {
+    pdl_enter();
+    if (ctl != nullptr && ctl->state != ST_RUNNING) return;
+    const int c = blockIdx.x * kMlWideThreads + threadIdx.x, plane = (int)g.plane;
+    if (c >= plane) return;
+    float H[NP], Lz[NP], Ip[NP];  // every plane's loads first (clamped addresses), then the sweeps
+#pragma unroll
+    for (int z = 0; z < NP; ++z) {
+        const int idx = (z < g.L ? z : g.L - 1) * plane + c;
         H[z] = R[idx];
         Lz[z] = lf[idx];
         Ip[z] = ipd[idx];
     }
     float gp = 0.f;
 #pragma unroll
-    for (int z = 0; z < NP; ++z) {
+    for (int z = 0; z < NP; ++z)
         if (z < g.L) {
-            const float gg = fmaf(-Lz[z], gp, H[z]);
-            H[z] = gg * fabsf(Ip[z]);
-            gp = gg;
+            gp = fmaf(-Lz[z], gp, H[z]);
+            H[z] = gp * fabsf(Ip[z]);
         }
-    }
     float wn = 0.f;
 #pragma unroll
-    for (int z = NP - 1; z >= 0; --z) {
+    for (int z = NP - 1; z >= 0; --z)
         if (z < g.L) {
             const float lup = (z + 1 < g.L) ? Lz[z + 1 < NP ? z + 1 : z] : 0.f;
             wn = fmaf(-lup, wn, H[z]);
-            xo[(long long)z * g.plane + c] = kMlOmega * wn;
+            xo[z * plane + c] = kMlOmega * wn;
         }
-    }
-}
-
-template <int NP>
-__global__ void __launch_bounds__(kMlThreads)
-    ml_presmooth(const float* __restrict__ R, float* __restrict__ xo, const float* __restrict__ lf,
-                 const float* __restrict__ ipd, MLGrid g, const SolveCtl* ctl) {
-    pdl_enter();
-    if (ctl != nullptr && ctl->state != ST_RUNNING) return;
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= g.plane) return;
-    ml_presmooth_column<NP>(R, xo, lf, ipd, g, c);
-}
-
-// Rc = Z^T (R - A x): the residual after pre-smoothing at every node, summed
-// over the non-empty nodes of each B x B aggregate (lanes x ^ 1 (, x ^ 2),
-// then the aggregate's B rows through shared memory).
-// The restriction of one 32 x 8 node tile (bx, by) of plane z: its partial
-// aggregate sums go through `s_part` (block shared memory, [8][kMlTile / B]);
-// the block's threads all take part.  A caller that runs several tiles in a
-// row must place a barrier between them.
-template <int B>
-__device__ __forceinline__ void ml_restrict_tile(const float* __restrict__ st, const float* __restrict__ R,
-                                                 const float* __restrict__ xv, const float* __restrict__ ipd,
-                                                 float* __restrict__ Rc, const MLGrid& g, const MLGrid& gc, int bx,
-                                                 int by, int z, float (*s_part)[kMlTile / B]) {
-    static_assert(B == 2 || B == 4, "aggregates are 2 x 2 or 4 x 4 node columns");
-    constexpr int AX_PER_BLOCK = kMlTile / B, AY_PER_BLOCK = 8 / B;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int x = bx * kMlTile + lane, y = by * 8 + warp;
-    float s = 0.f;
-    if (x < g.nx && y < g.ny) {
-        const long long idx = ml_index(g, z, y, x);
-        if (ipd[idx] >= 0.f)
-            s = R[idx] - (ml_interior(g, z, y, x) ? ml_stencil_dot<true>(st, xv, g, z, y, x)
-                                                  : ml_stencil_dot<false>(st, xv, g, z, y, x));
-    }
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    if (B == 4) s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if ((lane & (B - 1)) == 0) s_part[warp][lane / B] = s;
-    __syncthreads();
-    if (threadIdx.x < AX_PER_BLOCK * AY_PER_BLOCK) {
-        const int a_row = threadIdx.x / AX_PER_BLOCK, a_col = threadIdx.x % AX_PER_BLOCK;
-        const int AY = by * AY_PER_BLOCK + a_row, AX = bx * AX_PER_BLOCK + a_col;
-        if (AY < gc.ny && AX < gc.nx) {
-            const int w0 = B * a_row;
-            float v;
-            if (B == 4)
-                v = (s_part[w0][a_col] + s_part[w0 + 1][a_col]) + (s_part[w0 + 2][a_col] + s_part[w0 + 3][a_col]);
-            else
-                v = s_part[w0][a_col] + s_part[w0 + 1][a_col];
-            Rc[ml_index(gc, z, AY, AX)] = v;
-        }
-    }
-}
-
-template <int B>  // aggregate width g.b: 4 or 2
-__global__ void __launch_bounds__(kMlThreads)
-    ml_restrict(const float* __restrict__ st, const float* __restrict__ R, const float* __restrict__ xv,
-                const float* __restrict__ ipd, float* __restrict__ Rc, MLGrid g, MLGrid gc, const SolveCtl* ctl) {
-    __shared__ float s_part[8][kMlTile / B];
-    pdl_enter();
-    if (ctl != nullptr && ctl->state != ST_RUNNING) return;
-    ml_restrict_tile<B>(st, R, xv, ipd, Rc, g, gc, blockIdx.x, blockIdx.y, blockIdx.z, s_part);
-}
-
-// x += Z c on the non-empty nodes of a level (c: the correction of the level
-// below), before the level's residual.  One node column of kMlProlongPlanes
-// planes per thread (block z index = group of planes), every load issued
-// before the first store, so that a thread has several nodes' bytes in flight.
-constexpr int kMlProlongPlanes = 4;
-__device__ __forceinline__ void ml_prolong_column(float* __restrict__ xv, const float* __restrict__ cn,
-                                                  const float* __restrict__ ipd, const MLGrid& g, const MLGrid& gc,
-                                                  int z0, int y, int x) {
-    float xs[kMlProlongPlanes], cs[kMlProlongPlanes], ps[kMlProlongPlanes];
-#pragma unroll
-    for (int k = 0; k < kMlProlongPlanes; ++k) {
-        const int z = min(z0 + k, g.L - 1);  // clamped: valid addresses, stores guarded below
-        xs[k] = xv[ml_index(g, z, y, x)];
-        ps[k] = ipd[ml_index(g, z, y, x)];
-        cs[k] = cn[ml_index(gc, z, y / g.b, x / g.b)];
-    }
-#pragma unroll
-    for (int k = 0; k < kMlProlongPlanes; ++k)
-        if (z0 + k < g.L && ps[k] >= 0.f) xv[ml_index(g, z0 + k, y, x)] = xs[k] + cs[k];
-}
-
-__global__ void __launch_bounds__(kMlThreads)
-    ml_prolong(float* __restrict__ xv, const float* __restrict__ cn, const float* __restrict__ ipd, MLGrid g,
-               MLGrid gc, const SolveCtl* ctl) {
-    pdl_enter();
-    if (ctl != nullptr && ctl->state != ST_RUNNING) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int x = blockIdx.x * kMlTile + lane, y = blockIdx.y * 8 + warp;
-    if (x >= g.nx || y >= g.ny) return;
-    ml_prolong_column(xv, cn, ipd, g, gc, blockIdx.z * kMlProlongPlanes, y, x);
-}
-
-// t = R - A y' at every node (y' the prolonged x), written to `t` (the
-// level's output array, which ml_zsmooth then overwrites column by column).
-__device__ __forceinline__ void ml_residual_node(const float* __restrict__ st, const float* __restrict__ R,
-                                                 const float* __restrict__ xv, float* __restrict__ t,
-                                                 const MLGrid& g, int z, int y, int x) {
-    const long long idx = ml_index(g, z, y, x);
-    t[idx] = R[idx] - (ml_interior(g, z, y, x) ? ml_stencil_dot<true>(st, xv, g, z, y, x)
-                                               : ml_stencil_dot<false>(st, xv, g, z, y, x));
-}
-
-__global__ void __launch_bounds__(kMlThreads)
-    ml_residual(const float* __restrict__ st, const float* __restrict__ R, const float* __restrict__ xv,
-                float* __restrict__ t, MLGrid g, const SolveCtl* ctl) {
-    pdl_enter();
-    if (ctl != nullptr && ctl->state != ST_RUNNING) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int x = blockIdx.x * kMlTile + lane, y = blockIdx.y * 8 + warp, z = blockIdx.z;
-    if (x >= g.nx || y >= g.ny) return;
-    ml_residual_node(st, R, xv, t, g, z, y, x);
-}
-
-// Post-smoothing of column c: y = y' + omega T^-1 t with y' the prolonged x
-// and t from ml_residual (read from `yo` before it is overwritten there);
-// DOT: also acc += R.y over the column.
-template <int NP, bool DOT>
-__device__ __forceinline__ void ml_zsmooth_column(const float* __restrict__ R, const float* __restrict__ xv,
-                                                  const float* __restrict__ lf, const float* __restrict__ ipd,
-                                                  float* __restrict__ yo, const MLGrid& g, long long c, Acc32& acc) {
-    float H[NP], Lz[NP], Ip[NP];  // loads of every plane first (clamped addresses), then the sweeps
-#pragma unroll
-    for (int z = 0; z < NP; ++z) {
-        const long long idx = (long long)(z < g.L ? z : g.L - 1) * g.plane + c;
-        H[z] = yo[idx];
-        Lz[z] = lf[idx];
-        Ip[z] = ipd[idx];
-    }
-    float gp = 0.f;
-#pragma unroll
-    for (int z = 0; z < NP; ++z) {
-        if (z < g.L) {
-            const float gg = fmaf(-Lz[z], gp, H[z]);
-            H[z] = gg * fabsf(Ip[z]);
-            gp = gg;
-        }
-    }
-    float wn = 0.f;
-#pragma unroll
-    for (int z = NP - 1; z >= 0; --z) {
-        if (z < g.L) {
-            const long long idx = (long long)z * g.plane + c;
-            const float lup = (z + 1 < g.L) ? Lz[z + 1 < NP ? z + 1 : z] : 0.f;
-            wn = fmaf(-lup, wn, H[z]);
-            const float yv = fmaf(kMlOmega, wn, xv[idx]);
-            yo[idx] = yv;
-            if (DOT) acc.add_product(R[idx], yv);
-        }
-    }
-}
-
-// Post-smoothing, one column per thread (ml_zsmooth_column).  At the top level (MODE != ML_ONLY) the last block also
-// finishes r.z = r.T^-1 r + R.y and, for ML_ITER, beta and the iteration
-// limit; ML_START sets r.z.
-template <int NP, int MODE, bool TOP>
-__global__ void __launch_bounds__(kMlThreads)
-    ml_zsmooth(const float* __restrict__ R, const float* __restrict__ xv, const float* __restrict__ lf,
-               const float* __restrict__ ipd, float* __restrict__ yo, MLGrid g, SolveCtl* ctl, double* partials,
-               unsigned int* counter) {
-    __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc32) * 32];
-    Acc32* const scratch = reinterpret_cast<Acc32*>(scratch_raw);
-    pdl_enter();
-    if (MODE != ML_ONLY && ctl->state != ST_RUNNING) return;
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    Acc32 acc[1];
-    if (c < g.plane) ml_zsmooth_column<NP, TOP && MODE != ML_ONLY>(R, xv, lf, ipd, yo, g, c, acc[0]);
-    if (!TOP || MODE == ML_ONLY) return;
-    Acc32 tot[1];
-    if (ml_finish<1>(acc, scratch, partials, counter, tot)) {
-        const double rzn = ctl->rdr + tot[0].value();
-        if (MODE == ML_START) {
-            ctl->rz = rzn;
-        } else if (!isfinite(rzn) || ctl->rz == 0.0) {
-            ctl->state = ST_BREAKDOWN;
-        } else {
-            ctl->beta = rzn / ctl->rz;
-            ctl->rz = rzn;
-            if (ctl->iterations >= ctl->max_it) ctl->state = ST_MAXIT;
-        }
-    }
 }
 
 // ------------------------------------------------------------ set-up (FP64)
@@ -920,6 +1280,41 @@ __global__ void ml_coarsen(double* __restrict__ out, const double* __restrict__ 
         if (acc[0] == 0.0) acc[0] = -1.0;
 #pragma unroll
         for (int k = 0; k < kMlStencil; ++k) out[(long long)k * gc.n + I] = acc[k];
+    }
+}
+
+// A Z of a level (FP64 sums, stored FP32): per node i the entries A(i, j) of
+// its non-empty neighbours j summed by j's plane and by whether j lies in i's
+// aggregate row / column or in the one beside it (kMlAz arrays, plane major,
+// then row, then column); zero for an empty node.
+__global__ void ml_az(float* __restrict__ az, const double* __restrict__ in, MLGrid g) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < g.n; i += stride) {
+        const int z = (int)(i / g.plane);
+        const long long rem = i - (long long)z * g.plane;
+        const int y = (int)(rem / g.nx);
+        const int x = (int)(rem - (long long)y * g.nx);
+        double acc[kMlAz];
+#pragma unroll
+        for (int k = 0; k < kMlAz; ++k) acc[k] = 0.0;
+        if (!(in[i] < 0.0)) {
+#pragma unroll
+            for (int o = 0; o < 27; ++o) {
+                const int dz = o / 9 - 1, dy = (o / 3) % 3 - 1, dx = o % 3 - 1;
+                const int jz = z + dz, jy = y + dy, jx = x + dx;
+                if (jz < 0 || jz >= g.L || jy < 0 || jy >= g.ny || jx < 0 || jx >= g.nx) continue;
+                const long long j = ml_index(g, jz, jy, jx);
+                if (in[j] < 0.0) continue;  // empty
+                const double a = ml_coef(in, g.n, i, j, o);
+                const bool sy = jy / g.b != y / g.b, sx = jx / g.b != x / g.b;
+                acc[4 * (dz + 1) + 0] += (!sy && !sx) ? a : 0.0;
+                acc[4 * (dz + 1) + 1] += (!sy && sx) ? a : 0.0;
+                acc[4 * (dz + 1) + 2] += (sy && !sx) ? a : 0.0;
+                acc[4 * (dz + 1) + 3] += (sy && sx) ? a : 0.0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kMlAz; ++k) az[(long long)k * g.n + i] = (float)acc[k];
     }
 }
 

@@ -35,11 +35,9 @@ std::vector<MLGrid> ml_grids(const Layout& L) {
     return out;
 }
 
-// Fine pass: 32 x 8 node columns per block.  Coarse levels: one column per
-// thread (z-line kernels), one node per thread (residual kernels).
+// Fine pass: 32 x 8 node columns per block.  Coarse levels: 16 x 4 columns.
 dim3 ml_fine_grid(const Layout& L) { return dim3(ml_cdiv(L.Xp, kMlTile), ml_cdiv(L.R + 1, 8)); }
-dim3 ml_column_grid(const MLGrid& g) { return dim3((unsigned)((g.plane + kMlThreads - 1) / kMlThreads)); }
-dim3 ml_node_grid(const MLGrid& g) { return dim3(ml_cdiv(g.nx, kMlTile), ml_cdiv(g.ny, 8), g.L); }
+dim3 ml_level_grid(const MLGrid& g) { return dim3(ml_cdiv(g.nx, kMlColX), ml_cdiv(g.ny, kMlColY)); }
 
 void free_multilevel(tb_system* s) {
     dev_free(s, s->ml_zl);
@@ -52,6 +50,8 @@ void free_multilevel(tb_system* s) {
         dev_free(s, lv.lf);
         dev_free(s, lv.ipd);
         dev_free(s, lv.x);
+        dev_free(s, lv.az);
+        dev_free(s, lv.s);
         if (l + 1 < c) {  // the coarsest level's R and y are coarse_rc and coarse_c
             dev_free(s, lv.R);
             dev_free(s, lv.y);
@@ -96,59 +96,129 @@ cudaError_t launch_coarse_apply(tb_system* s, bool pdl) {
 }
 
 template <typename... KArgs, typename... Args>
-cudaError_t ml_launch(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t stream, Args... args) {
-    if (pdl) return launch_pdl(kernel, grid, block, 0, stream, args...);
-    kernel<<<grid, block, 0, stream>>>(static_cast<KArgs>(args)...);
+cudaError_t ml_launch_smem(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                           Args... args) {
+    if (pdl) return launch_pdl(kernel, grid, block, smem, stream, args...);
+    kernel<<<grid, block, smem, stream>>>(static_cast<KArgs>(args)...);
     return cudaGetLastError();
 }
+template <typename... KArgs, typename... Args>
+cudaError_t ml_launch(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t stream, Args... args) {
+    return ml_launch_smem(pdl, kernel, grid, block, 0, stream, args...);
+}
 
-int ml_vcycle_kernels(const tb_system* s) {
-    const int c = (int)s->ml.size();
-    return c <= 1 ? 1 : 5 * (c - 1) + 1;
+// Node columns from which a level runs with one thread per column (the wide
+// forms), and from which level 1's pre-smoothing is a kernel of its own
+// instead of the tail of the fine pass's blocks.  Microseconds per iteration
+// on c3 boards of 256 .. 2048 cells a side (level 1: 4,225 .. 263,169 columns),
+// node form / wide form of one step, the other two unchanged:
+//   columns        16,641         25,921         37,249         51,076         66,049
+//   ml_down   121.1 / 134.0  166.4 / 174.5  221.0 / 224.1  313.4 / 321.7  388.0 / 390.7
+//   ml_up     121.1 / 125.9  166.4 / 169.3  221.0 / 220.8  313.4 / 306.8  388.0 / 372.8
+//   pre       121.1 / 121.6  166.4 / 165.9  221.0 / 216.4  313.4 / 307.9  388.0 / 380.3
+// and on 2048 cells ml_down of level 1 118 / 108 us, ml_up 160 / 85 us, the
+// fine pass 397 us with the pre-smoothing in its blocks against 344 + 14 us.
+constexpr long long kMlWideDown = 130000, kMlWideUp = 40000, kMlWidePre = 25000;
+bool ml_wide_down(const MLGrid& g) { return g.plane >= kMlWideDown; }
+bool ml_wide_up(const MLGrid& g) { return g.plane >= kMlWideUp; }
+bool ml_wide_pre(const tb_system* s) { return s->ml.size() > 1 && s->ml[0].g.plane >= kMlWidePre; }
+dim3 ml_column_grid(const MLGrid& g) { return dim3((unsigned)((g.plane + kMlWideThreads - 1) / kMlWideThreads)); }
+
+int ml_vcycle_kernels(const tb_system* s) { return 2 * (int)s->ml.size() - 1 + (ml_wide_pre(s) ? 1 : 0); }
+
+// The level's pre-smoothing is done by the kernel that forms its right-hand
+// side; the densely inverted grid has none.
+MLNext ml_next(const tb_system* s) {
+    if (s->ml.size() <= 1 || ml_wide_pre(s)) return MLNext{nullptr, nullptr, nullptr};
+    return MLNext{s->ml[0].lf, s->ml[0].ipd, s->ml[0].x};
+}
+
+// ml_down loads its coefficients ahead of the dependency wait on grids of at
+// most kMlPreBlocks blocks per SM: beyond that blocks start after the wait has
+// passed, and its 96 registers leave one block per SM.  c2 (297 blocks on level
+// 1): 100.3 us per iteration with 4, 96.4 with 1; a 71 x 93 board (12 blocks):
+// 33.0 us without the early loads, 30.9 with them.
+constexpr int kMlPreBlocks = 1;
+
+template <int B, int ROUNDS>
+cudaError_t ml_launch_down(tb_system* s, int l, bool pdl, const SolveCtl* ctl) {
+    constexpr bool CAN = ROUNDS <= kMlPreRounds;
+    const tb_system::MLLevel& lv = s->ml[l];
+    const tb_system::MLLevel& dn = s->ml[l + 1];
+    const bool dense = l + 2 == (int)s->ml.size();
+    const dim3 grid = ml_level_grid(lv.g);
+    if (ml_wide_down(lv.g)) {
+        constexpr int NP = ROUNDS == 1 ? 9 : (ROUNDS == 2 ? 18 : 33);
+        return ml_launch(pdl, ml_down_wide<NP, B>, dim3(ml_cdiv(lv.g.nx, kMlWideX), ml_cdiv(lv.g.ny, kMlWideY)),
+                         dim3(kMlWideThreads), s->stream, (const float*)lv.st, (const float*)lv.R, (const float*)lv.x,
+                         (const float*)lv.ipd, lv.s, dn.R, dense ? (float*)nullptr : dn.x, (const float*)dn.lf,
+                         (const float*)dn.ipd, lv.g, dn.g, ctl);
+    }
+    const bool pre = CAN && (int)(grid.x * grid.y) <= kMlPreBlocks * s->sms;
+    return ml_launch_smem(pdl, pre ? ml_down<B, ROUNDS, CAN> : ml_down<B, ROUNDS, false>, grid,
+                          dim3(kMlCols * ml_level_groups(lv.g.L)), ml_level_smem(lv.g.L), s->stream,
+                          (const float*)lv.st, (const float*)lv.R, (const float*)lv.x, (const float*)lv.ipd, lv.s,
+                          dn.R, dense ? (float*)nullptr : dn.x, (const float*)dn.lf, (const float*)dn.ipd, lv.g, dn.g,
+                          ctl);
+}
+
+template <int B>
+cudaError_t ml_launch_down(tb_system* s, int l, bool pdl, const SolveCtl* ctl) {
+    const int rounds = ml_level_rounds(s->ml[l].g.L);
+    if (rounds == 1) return ml_launch_down<B, 1>(s, l, pdl, ctl);
+    if (rounds == 2) return ml_launch_down<B, 2>(s, l, pdl, ctl);
+    return ml_launch_down<B, 4>(s, l, pdl, ctl);
+}
+
+template <int B, int ROUNDS>
+cudaError_t ml_launch_up(tb_system* s, int l, int mode, bool pdl) {
+    const tb_system::MLLevel& lv = s->ml[l];
+    const tb_system::MLLevel& dn = s->ml[l + 1];
+    SolveCtl* const state = mode == ML_ONLY ? nullptr : s->ctl;
+    if (ml_wide_up(lv.g)) {
+        constexpr int NP = ROUNDS == 1 ? 9 : (ROUNDS == 2 ? 18 : 33);
+        return ml_launch(pdl, l == 0 ? ml_up_wide<NP, B, true> : ml_up_wide<NP, B, false>,
+                         ml_column_grid(lv.g), dim3(kMlWideThreads), s->stream, (const float*)lv.az,
+                         (const float*)lv.R, (const float*)lv.s, (const float*)lv.x, (const float*)dn.y,
+                         (const float*)lv.lf, (const float*)lv.ipd, lv.y, lv.g, dn.g, state, mode,
+                         s->partials, s->counter);
+    }
+    return ml_launch_smem(pdl, l == 0 ? ml_up<B, ROUNDS, true> : ml_up<B, ROUNDS, false>,
+                          ml_level_grid(lv.g), dim3(kMlCols * ml_level_groups(lv.g.L)), ml_level_smem(lv.g.L),
+                          s->stream, (const float*)lv.az, (const float*)lv.R, (const float*)lv.s, (const float*)lv.x,
+                          (const float*)dn.y, (const float*)lv.lf, (const float*)lv.ipd, lv.y, lv.g, dn.g, state,
+                          mode, s->partials, s->counter);
+}
+template <int B>
+cudaError_t ml_launch_up(tb_system* s, int l, int mode, bool pdl) {
+    const int rounds = ml_level_rounds(s->ml[l].g.L);
+    if (rounds == 1) return ml_launch_up<B, 1>(s, l, mode, pdl);
+    if (rounds == 2) return ml_launch_up<B, 2>(s, l, mode, pdl);
+    return ml_launch_up<B, 4>(s, l, mode, pdl);
 }
 
 // One preconditioner action after the fine pass: the V-cycle over the coarse
 // levels (MODE: ML_ITER / ML_START finish r.z at the top, ML_ONLY does not).
-template <int NP, int MODE>
+template <int MODE>
 cudaError_t ml_vcycle(tb_system* s, bool pdl) {
     const int c = (int)s->ml.size();
     if (c == 1) {
         constexpr int CM = (MODE == ML_ITER) ? COARSE_ITERATE : (MODE == ML_START ? COARSE_START : COARSE_ONLY);
         return launch_coarse_apply<CM>(s, pdl);
     }
-    SolveCtl* ctl = (MODE == ML_ONLY) ? nullptr : s->ctl;
+    const SolveCtl* ctl = (MODE == ML_ONLY) ? nullptr : s->ctl;
     cudaError_t e = cudaSuccess;
-    for (int l = 0; l + 1 < c && e == cudaSuccess; ++l) {
-        const tb_system::MLLevel& lv = s->ml[l];
-        const tb_system::MLLevel& dn = s->ml[l + 1];
-        e = ml_launch(pdl, ml_presmooth<NP>, ml_column_grid(lv.g), dim3(kMlThreads), s->stream, (const float*)lv.R,
-                      lv.x, (const float*)lv.lf, (const float*)lv.ipd, lv.g, (const SolveCtl*)ctl);
-        if (e == cudaSuccess)
-            e = ml_launch(pdl, lv.g.b == 4 ? ml_restrict<4> : ml_restrict<2>, ml_node_grid(lv.g), dim3(kMlThreads),
-                          s->stream, (const float*)lv.st, (const float*)lv.R, (const float*)lv.x,
-                          (const float*)lv.ipd, dn.R, lv.g, dn.g, (const SolveCtl*)ctl);
+    if (ml_wide_pre(s)) {
+        const tb_system::MLLevel& lv = s->ml[0];
+        e = ml_launch(pdl, lv.g.L <= 9 ? ml_presmooth<9> : (lv.g.L <= 17 ? ml_presmooth<17> : ml_presmooth<33>),
+                      ml_column_grid(lv.g), dim3(kMlWideThreads), s->stream, (const float*)lv.R, lv.x,
+                      (const float*)lv.lf, (const float*)lv.ipd, lv.g, ctl);
     }
+    for (int l = 0; l + 1 < c && e == cudaSuccess; ++l)
+        e = s->ml[l].g.b == 4 ? ml_launch_down<4>(s, l, pdl, ctl) : ml_launch_down<2>(s, l, pdl, ctl);
     if (e == cudaSuccess) e = launch_coarse_apply<COARSE_ONLY>(s, pdl);
-    for (int l = c - 2; l >= 0 && e == cudaSuccess; --l) {
-        const tb_system::MLLevel& lv = s->ml[l];
-        const tb_system::MLLevel& dn = s->ml[l + 1];
-        e = ml_launch(pdl, ml_prolong,
-                      dim3(ml_cdiv(lv.g.nx, kMlTile), ml_cdiv(lv.g.ny, 8), ml_cdiv(lv.g.L, kMlProlongPlanes)),
-                      dim3(kMlThreads), s->stream, lv.x, (const float*)dn.y,
-                      (const float*)lv.ipd, lv.g, dn.g, (const SolveCtl*)ctl);
-        if (e == cudaSuccess)
-            e = ml_launch(pdl, ml_residual, ml_node_grid(lv.g), dim3(kMlThreads), s->stream, (const float*)lv.st,
-                          (const float*)lv.R, (const float*)lv.x, lv.y, lv.g, (const SolveCtl*)ctl);
-        if (e != cudaSuccess) break;
-        if (l == 0)
-            e = ml_launch(pdl, ml_zsmooth<NP, MODE, true>, ml_column_grid(lv.g), dim3(kMlThreads), s->stream,
-                          (const float*)lv.R, (const float*)lv.x, (const float*)lv.lf, (const float*)lv.ipd, lv.y,
-                          lv.g, ctl, s->partials, s->counter);
-        else
-            e = ml_launch(pdl, ml_zsmooth<NP, MODE, false>, ml_column_grid(lv.g), dim3(kMlThreads), s->stream,
-                          (const float*)lv.R, (const float*)lv.x, (const float*)lv.lf, (const float*)lv.ipd, lv.y,
-                          lv.g, ctl, s->partials, s->counter);
-    }
+    for (int l = c - 2; l >= 0 && e == cudaSuccess; --l)
+        e = s->ml[l].g.b == 4 ? ml_launch_up<4>(s, l, MODE, pdl) : ml_launch_up<2>(s, l, MODE, pdl);
     return e;
 }
 
@@ -221,18 +291,19 @@ cudaError_t ml_fine_pass(tb_system* s, bool pdl) {
         const size_t smem = ml_stage_smem(s->lay, s->ml_stages);
         if (pdl)
             return launch_pdl(ml_update_staged<NP>, dim3(grid), dim3(kMlThreads), smem, s->stream, s->r32, s->ml_w,
-                              s->ml[0].R, s->lay, s->pstride, s->ml[0].g, s->ctl, s->partials, s->counter,
-                              s->clocks + 2, (int)tg.x, tiles, s->ml_stages, s->ml_maps);
+                              s->ml[0].R, s->lay, s->pstride, s->ml[0].g, ml_next(s), s->ctl, s->partials,
+                              s->counter, s->clocks + 2, (int)tg.x, tiles, s->ml_stages, s->ml_maps);
         ml_update_staged<NP><<<grid, kMlThreads, smem, s->stream>>>(s->r32, s->ml_w, s->ml[0].R, s->lay, s->pstride,
-                                                                     s->ml[0].g, s->ctl, s->partials, s->counter,
+                                                                     s->ml[0].g, ml_next(s), s->ctl, s->partials,
+                                                                     s->counter,
                                                                      s->clocks + 2, (int)tg.x, tiles, s->ml_stages,
                                                                      s->ml_maps);
         return cudaGetLastError();
     }
     return ml_launch(pdl, ml_update<NP, MODE>, ml_fine_grid(s->lay), dim3(kMlThreads), s->stream, s->r32,
                      (const float*)s->q32, (const double*)s->r64, s->x32, s->ml_w, s->ml[0].R, (const float*)s->ml_zl,
-                     (const float*)s->ml_zi, s->lay, s->pstride, s->ml[0].g, s->ctl, s->partials, s->counter,
-                     s->clocks + 2);
+                     (const float*)s->ml_zi, s->lay, s->pstride, s->ml[0].g, ml_next(s), s->ctl, s->partials,
+                     s->counter, s->clocks + 2);
 }
 
 template <bool START>
@@ -249,15 +320,15 @@ cudaError_t ml_step_np(tb_system* s, int mode, bool pdl) {
     cudaError_t e;
     if (mode == ML_ITER) {
         e = ml_fine_pass<NP, ML_ITER>(s, pdl);
-        if (e == cudaSuccess) e = ml_vcycle<NP, ML_ITER>(s, pdl);
+        if (e == cudaSuccess) e = ml_vcycle<ML_ITER>(s, pdl);
         if (e == cudaSuccess) e = ml_launch_direction<false>(s, pdl, s->ctl);
     } else if (mode == ML_START) {
         e = ml_fine_pass<NP, ML_START>(s, pdl);
-        if (e == cudaSuccess) e = ml_vcycle<NP, ML_START>(s, pdl);
+        if (e == cudaSuccess) e = ml_vcycle<ML_START>(s, pdl);
         if (e == cudaSuccess) e = ml_launch_direction<true>(s, pdl, s->ctl);
     } else {
         e = ml_fine_pass<NP, ML_ONLY>(s, pdl);
-        if (e == cudaSuccess) e = ml_vcycle<NP, ML_ONLY>(s, pdl);
+        if (e == cudaSuccess) e = ml_vcycle<ML_ONLY>(s, pdl);
         if (e == cudaSuccess) e = ml_launch_direction<true>(s, pdl, nullptr);
     }
     return e;
@@ -271,7 +342,7 @@ cudaError_t ml_step64_np(tb_system* s, bool start, bool pdl) {
     cudaError_t e;
     if (start) {
         e = ml_fine_pass<NP, ML_START>(s, pdl);
-        if (e == cudaSuccess) e = ml_vcycle<NP, ML_START>(s, pdl);
+        if (e == cudaSuccess) e = ml_vcycle<ML_START>(s, pdl);
         if (e == cudaSuccess)
             e = ml_launch(pdl, ml_direction_f64<true>, vg, vb, s->stream, s->p64, (const float*)s->ml_w,
                           (const float*)s->ml[0].y, (const float*)s->ml_zi, s->nq, s->lay, s->ml[0].g, s->special_mask,
@@ -279,7 +350,7 @@ cudaError_t ml_step64_np(tb_system* s, bool start, bool pdl) {
         return e;
     }
     e = ml_fine_pass<NP, ML_PRE64>(s, pdl);
-    if (e == cudaSuccess) e = ml_vcycle<NP, ML_ITER>(s, pdl);
+    if (e == cudaSuccess) e = ml_vcycle<ML_ITER>(s, pdl);
     if (e == cudaSuccess)
         e = ml_launch(pdl, ml_direction_f64<false>, vg, vb, s->stream, s->p64, (const float*)s->ml_w,
                       (const float*)s->ml[0].y, (const float*)s->ml_zi, s->nq, s->lay, s->ml[0].g, s->special_mask,
@@ -352,6 +423,8 @@ int build_multilevel(tb_system* s) {
             TB_CHECK(alloc_n(s, &lv.st, kMlStencil * n));
             TB_CHECK(alloc_n(s, &lv.lf, n));
             TB_CHECK(alloc_n(s, &lv.ipd, n));
+            TB_CHECK(alloc_n(s, &lv.az, kMlAz * n));
+            TB_CHECK(alloc_n(s, &lv.s, n));
             TB_CHECK(alloc_n(s, &lv.R, n));
             TB_CHECK(alloc_n(s, &lv.y, n));
         } else {
@@ -401,12 +474,13 @@ int build_multilevel(tb_system* s) {
         for (int l = 0; l + 1 < c; ++l) {
             tb_system::MLLevel& lv = s->ml[l];
             ml_level_factors<<<grid_for(lv.g.plane, 128, sb), 128, 0, st>>>(lv.st, lv.lf, lv.ipd, st64[l], lv.g);
+            ml_az<<<grid_for(lv.g.n, 128, sb), 128, 0, st>>>(lv.az, st64[l], lv.g);
         }
         cudaMemsetAsync(s->coarse_matrix, 0, sizeof(double) * nn, st);
         ml_dense<<<grid_for(nc, 128, sb), 128, 0, st>>>(s->coarse_matrix, st64[c - 1], gc);
         cudaMemcpyAsync(work, s->coarse_matrix, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st);
         cudaMemsetAsync(s->d_err, 0, sizeof(int), st);
-        s->kernel_launches += 2 + 2 * (c - 1);
+        s->kernel_launches += 2 + 3 * (c - 1);
         check_launch();
     }
     if (rc == TB_OK && gauss_jordan_invert(work, cl.nc, s->d_err, st) != cudaSuccess)
@@ -435,8 +509,8 @@ int build_multilevel(tb_system* s) {
     const int planes = L.S + 1;
     s->ml_np = planes <= 9 ? 9 : (planes <= 17 ? 17 : 33);
     {
-        const dim3 fg = ml_fine_grid(L), tg = ml_column_grid(grids[0]);
-        TB_CHECK(ensure_partials(s, std::max((int)(fg.x * fg.y), (int)tg.x)));
+        const dim3 fg = ml_fine_grid(L), tg = ml_level_grid(grids[0]);  // the widest of the level forms
+        TB_CHECK(ensure_partials(s, (int)std::max(fg.x * fg.y, tg.x * tg.y)));
     }
     TB_CHECK(ml_stage_setup(s));
     return keep_coarse_in_l2(s);

@@ -162,6 +162,7 @@ struct tb_system {
     struct MLLevel {
         MLGrid g{};
         float *st = nullptr, *lf = nullptr, *ipd = nullptr, *R = nullptr, *x = nullptr, *y = nullptr;
+        float *az = nullptr, *s = nullptr;  // A Z (kMlAz arrays) and the pre-smoothed residual
     };
     float *ml_zl = nullptr, *ml_zi = nullptr, *ml_w = nullptr;
     std::vector<MLLevel> ml;
