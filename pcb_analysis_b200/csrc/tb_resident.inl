@@ -1,0 +1,148 @@
+// Host side of the cooperative PCG kernel of small boards (tb_resident.cuh).
+// Included by tb_system.cu inside its anonymous namespace.
+
+constexpr int kResLimit = 512;      // iterations of one launch (a few milliseconds)
+constexpr int kResMinChunk = 128;   // nodes of a block at least
+
+using ResidentKernel = void (*)(const ResidentParams);
+ResidentKernel resident_kernel(int nodes, bool tl) {
+    if (nodes == 1) return tl ? resident_pcg<1, true> : resident_pcg<1, false>;
+    return tl ? resident_pcg<2, true> : resident_pcg<2, false>;
+}
+
+void free_resident(tb_system* s) {
+    dev_free(s, s->res_rows);
+    dev_free(s, s->res_words);
+    s->res_state = 0;
+}
+
+// Whether the system's inner PCG runs as the cooperative kernel, and its
+// buffers: thermal systems with the Jacobi or two-level preconditioner whose
+// nodes fit the registers of one block per SM (two nodes a thread) and, with
+// the coarse inverse's tile, its shared memory.  A launch plan set
+// by the caller (tb_set_apply_plan) and event timing (tb_set_timing) ask for
+// the graph-captured kernels.
+int resident_setup(tb_system* s) {
+    if (s->res_state != 0) return TB_OK;
+    s->res_state = -1;  // not available
+    const Layout& L = s->lay;
+    const bool tl = s->precond == 1;
+    if (s->physics != 0 || s->precond > 1 || s->sms > kResMaxBlocks) return TB_OK;
+    if (L.L > (long long)s->sms * kResThreads * kResNodes) return TB_OK;
+    int coop = 0;
+    TB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
+    if (!coop) return TB_OK;
+    const int chunk = std::max(kResMinChunk, (int)round_up((L.L + s->sms - 1) / s->sms, 32));
+    const int blocks = (int)((L.L + chunk - 1) / chunk);
+    // tiles of the inverse: as square as the blocks allow
+    const int tiles_y = tl ? std::max(1, (int)std::sqrt((double)blocks)) : 0;
+    const int tiles_x = tl ? std::min(blocks / tiles_y, kResTileCols) : 0;
+    const int trows = tl ? (int)round_up((s->cl.nc + tiles_y - 1) / tiles_y, 4) : 0;
+    const int tcols = tl ? (int)round_up((s->cl.nc + tiles_x - 1) / tiles_x, 4) : 0;
+    if (trows + tcols > kResThreads) return TB_OK;
+    const int nodes = chunk <= kResThreads ? 1 : 2;
+    const size_t smem = resident_smem(trows, tcols, chunk, L.Xp);
+    int optin = 0;
+    TB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
+    const ResidentKernel kernel = resident_kernel(nodes, tl);
+    cudaFuncAttributes fa{};
+    TB_CUDA(cudaFuncGetAttributes(&fa, kernel));
+    if (fa.sharedSizeBytes + smem > (size_t)optin) return TB_OK;
+    TB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 optin - (int)fa.sharedSizeBytes));
+    int per_sm = 0;
+    TB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kResThreads, smem));
+    if (per_sm < 1) return TB_OK;
+    int slots = 0;
+    if (tl) {
+        // blocks that touch one patch row: from the one that holds its first node on
+        const int prows = s->cl.layers * s->cl.nby;
+        for (int pr = 0; pr < prows; ++pr) {
+            const int z = pr / s->cl.nby, y0 = (pr - z * s->cl.nby) * s->cl.b;
+            const long long first = ((long long)z * (L.R + 1) + y0) * L.Xp;
+            const long long last = first + (long long)std::min(s->cl.b, L.R + 1 - y0) * L.Xp - 1;
+            slots = std::max(slots, (int)(last / chunk - first / chunk) + 1);
+        }
+        // patch rows one block touches: a chunk spans at most chunk / Xp + 2 lines,
+        // and a patch row has b of them except at the end of a plane
+        const int lines = chunk / L.Xp + 2;
+        const int touched = std::min(prows, lines / s->cl.b + lines / (L.R + 1) + 3) * s->cl.nbx;
+        if (slots > kResSlots || touched > kResTouched) return TB_OK;
+    }
+    TB_CHECK(alloc_n(s, &s->res_rows, kResRow * L.L));
+    // tagged words: the direction, the sums, the patch sums, the coarse solution; and the next tag
+    const long long sums = 8LL * kResCopies * blocks, parts = tl ? (long long)slots * s->cl.ld : 0, cs = (long long)tiles_x * s->cl.ld;
+    s->res_word_count = L.L + sums + parts + cs + 1;  // L is a multiple of 4: the sums' pairs stay 16-byte aligned
+    TB_CHECK(alloc_n(s, &s->res_words, s->res_word_count));
+    resident_rows<<<grid_for(L.L, 128, s->sms * 16), 128, 0, s->stream>>>(
+        s->res_rows, s->kin64, s->kz64, s->rf64, s->dims64, s->dims64 + L.S, s->dims64 + L.S + L.C, L);
+    TB_CUDA(cudaGetLastError());
+    s->kernel_launches += 1;
+    ResidentParams P{};
+    P.p = s->p32;
+    P.x = s->x32;
+    P.r = s->r32;
+    P.dinv = s->dinv32;
+    P.halo = s->res_words;
+    P.rows = s->res_rows;
+    P.lay = L;
+    P.pstride = (int)s->pstride;
+    P.ctl = s->ctl;
+    P.clock = s->clocks;
+    P.posts = P.halo + L.L;
+    P.part = P.posts + sums;
+    P.c = P.part + parts;
+    P.tag = reinterpret_cast<unsigned int*>(P.c + cs);
+    P.err = s->stage_err;
+    P.chunk = chunk;
+    P.limit = kResLimit;
+    P.polls = kResPolls;
+    P.cl = s->cl;
+    P.minv = tl ? s->coarse_inv32 : nullptr;
+    P.slots = slots;
+    P.tiles_x = tiles_x;
+    P.tiles_y = tiles_y;
+    P.trows = trows;
+    P.tcols = tcols;
+    s->res_params = P;
+    s->res_blocks = blocks;
+    s->res_nodes = nodes;
+    s->res_smem = smem;
+    s->res_fresh = true;
+    s->res_state = 1;
+    return TB_OK;
+}
+
+bool resident_wanted(const tb_system* s) { return !s->timing && !s->plan_set && s->physics == 0 && s->precond <= 1; }
+
+// The inner PCG from a prepared start (as run_pcg) on the cooperative kernel.
+int run_resident(tb_system* s, SolveCtl* out) {
+    if (s->res_fresh) {  // nothing exchanged yet, or a run that was given up: words without tags, the first tag 1
+        TB_CUDA(cudaMemsetAsync(s->res_words, 0, sizeof(unsigned long long) * (size_t)s->res_word_count, s->stream));
+        const unsigned int first = 1;
+        TB_CUDA(cudaMemcpyAsync(s->res_params.tag, &first, sizeof(first), cudaMemcpyHostToDevice, s->stream));
+        TB_CUDA(cudaStreamSynchronize(s->stream));
+        s->res_fresh = false;
+    }
+    ResidentParams P = s->res_params;
+    if (s->maps[0].test_polls > 0) {
+        P.polls = s->maps[0].test_polls;
+        P.mute = 1;
+    }
+    const ResidentKernel kernel = resident_kernel(s->res_nodes, P.minv != nullptr);
+    void* args[] = {&P};
+    for (long long n = 0;; ++n) {
+        TB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(s->res_blocks),
+                                            dim3(kResThreads), args, s->res_smem, s->stream));
+        s->kernel_launches += 1;
+        TB_CHECK(read_ctl(s, out));
+        if (out->state != ST_RUNNING) break;
+        if (n > (1LL << 40)) return fail(TB_ETIMEOUT, "PCG did not stop");
+    }
+    if (out->state == ST_STAGE_TIMEOUT) {
+        s->res_fresh = true;
+        return check_stage(s) == TB_OK ? fail(TB_ETIMEOUT, "a block of the PCG kernel gave up waiting for the others")
+                                       : TB_ETIMEOUT;
+    }
+    return TB_OK;
+}

@@ -36,6 +36,7 @@
 #include "tb_multilevel.cuh"
 #include "tb_prep.cuh"
 #include "tb_reduce.cuh"
+#include "tb_resident.cuh"
 #include "tb_types.h"
 #include "tb_vec.cuh"
 #include "tb_warp_apply.cuh"
@@ -176,6 +177,16 @@ struct tb_system {
     // the plain FP64 PCG preconditioned by the multilevel operator (set for
     // the call of tb_solve_pcg_f64_ml*), and the kind the FP64 graphs hold
     bool pcg64_ml = false, slots64_ml = false;
+    // the cooperative PCG kernel of small boards (tb_resident.inl): 0 not set
+    // up, 1 ready, -1 not available; its operator rows and tagged words
+    int res_state = 0, res_blocks = 0, res_nodes = 0;
+    size_t res_smem = 0;
+    bool res_fresh = true;
+    bool plan_set = false;  // the caller chose the operator's launch plan
+    float* res_rows = nullptr;
+    unsigned long long* res_words = nullptr;
+    long long res_word_count = 0;
+    ResidentParams res_params{};
     // problem terms of a system made by tb_system_create_problem (flat node
     // order): node flags, loads, Robin terms, C / dt, fixed values, and each
     // convection boundary's lumped weights for its removed heat
@@ -842,6 +853,8 @@ int accumulate_chunk(tb_system* s, const ChunkSlot& slot, int worked, bool f64) 
 
 int check_stage(tb_system* s);
 
+#include "tb_resident.inl"
+
 int kernels_per_iteration(const tb_system* s, bool f64) {
     if (f64 && s->pcg64_ml) return 2 + ml_kernels_per_step(s);
     if (!f64 && s->precond == 2) return 1 + ml_kernels_per_step(s);
@@ -858,6 +871,10 @@ int kernels_per_iteration(const tb_system* s, bool f64) {
 // wrong guess costs one host round trip; the iterations themselves, and so
 // the results, do not depend on it.
 int run_pcg(tb_system* s, bool f64, SolveCtl* out) {
+    if (!f64 && resident_wanted(s)) {
+        TB_CHECK(resident_setup(s));
+        if (s->res_state == 1) return run_resident(s, out);
+    }
     TB_CHECK(ensure_slots(s, f64));
     ChunkSlot* slots = f64 ? s->slots64 : s->slots32;
     SolveCtl start;
@@ -1617,6 +1634,7 @@ int set_preconditioner(tb_system* s, int kind, int block) {
         release_slot(s->slots64[k]);
     }
     s->precond = 0;
+    free_resident(s);
     free_multilevel(s);
     if (kind == 0) {
         free_coarse(s);
@@ -1663,6 +1681,7 @@ int refresh_robin(tb_system* s, const double* d_robin) {
         release_slot(s->slots64[k]);
     }
     if (s->special_mask != old_mask) TB_CHECK(autotune_tile(s));
+    free_resident(s);  // its operator rows hold the old Robin totals
     if (s->precond == 1) TB_CHECK(set_preconditioner(s, 1, s->cl.b));
     if (s->precond == 2) TB_CHECK(set_preconditioner(s, 2, 0));
     return TB_OK;
@@ -2600,6 +2619,7 @@ int tb_set_apply_plan(tb_system* s, const int32_t* plan5) {
     TB_CUDA(cudaSetDevice(s->device));
     TB_CUDA(cudaStreamSynchronize(s->stream));
     s->plan = p;
+    s->plan_set = true;
     for (int k = 0; k < 2; ++k) {  // captured chunks hold the old launch shape
         release_slot(s->slots32[k]);
         release_slot(s->slots64[k]);

@@ -1,0 +1,138 @@
+"""The cooperative PCG kernel of small boards against the graph-captured kernels.
+
+A launch plan set by the caller selects the graph-captured kernels, so each
+solve runs both ways: the same stopping rules on the same FP32 recurrences,
+rounded differently.  Tolerances: two converged refinements (FP64 residual
+1e-10) agree like any two of them, 1e-7 of the peak rise; the residual one
+inner solve can attain in FP32 is within a factor of two.  Iteration counts are
+not compared: an inner residual that lingers above its tolerance crosses it
+hundreds of iterations apart in two roundings (the graph-captured plans among
+themselves: 4,220 and 4,637 on one of these boards).
+"""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from pcb_analysis_b200 import workloads
+from pcb_analysis_b200.mpir import MPIRConfig
+
+pytestmark = pytest.mark.gpu
+
+CONFIG = MPIRConfig(inner_relative_tolerance=1e-3, max_outer_iterations=40, max_inner_iterations=100000)
+
+
+def _board(ns, slabs, rows, cols, fixed, void):
+    rng = np.random.default_rng(rows + 7 * cols + slabs)
+    k = np.full((slabs, rows, cols), 0.3)
+    for z in range(0, slabs, 3):
+        k[z] = np.where(rng.random((rows, cols)) < 0.6, 385.0, 0.3)
+    kwargs = {}
+    if void:
+        active = np.ones((slabs, rows, cols), dtype=bool)
+        active[:, rows // 2 :, cols // 2 :] = False
+        kwargs["active"] = active
+    mesh = ns.LayeredThermalMesh(
+        slab_thickness_m=tuple(35e-6 if z % 3 == 0 else 0.3e-3 for z in range(slabs)),
+        pitch_x_m=np.linspace(0.2e-3, 0.3e-3, cols), pitch_y_m=0.25e-3, conductivity_w_per_m_k=k,
+        through_plane_conductivity_w_per_m_k=0.5 * k, **kwargs)
+    problem = {}
+    if fixed:
+        mask = np.zeros(mesh.node_shape, dtype=bool)
+        mask[0, :, 0] = True
+        problem = dict(fixed_temperature_mask=mask, fixed_temperature_k=310.0)
+    return ns.ThermalConductionProblem(
+        mesh, convection=(ns.ConvectionBoundary("top", 12.0, 298.15),),
+        heat_sources=(ns.HeatSource(((slabs, rows // 3, cols // 3),), 0.2),), **problem)
+
+
+def _both(ns, problem, preconditioner, config):
+    out = []
+    for graph in (False, True):
+        op = ns.MatrixFreeThermalOperator(problem, preconditioner=preconditioner)
+        try:
+            if graph:
+                op.device_system.apply_plan = op.device_system.apply_plan
+            rhs = op.build_rhs(op.default_reference_temperature())
+            launches = op.device_system.launch_count()
+            out.append(op.device_system.solve_mpir(rhs, config) | {"rhs": rhs})
+            out[-1]["launches"] = op.device_system.launch_count() - launches
+        finally:
+            op.close()
+    return out
+
+
+@pytest.mark.parametrize("preconditioner", ["jacobi", "two-level"])
+@pytest.mark.parametrize(
+    "slabs, rows, cols, fixed, void",
+    [
+        (1, 1, 1, False, False),      # one element: one block
+        (2, 9, 130, True, False),     # rows longer than a block's nodes
+        (5, 37, 44, False, True),     # void elements: rows without an unknown
+        (8, 100, 101, True, False),   # one node per thread
+        (8, 128, 128, False, False),  # two nodes per thread
+        (12, 118, 127, True, True),   # near the largest board the kernel takes
+    ],
+)
+def test_small_boards_solve_alike(ns_local, preconditioner, slabs, rows, cols, fixed, void):
+    one, graph = _both(ns_local, _board(ns_local, slabs, rows, cols, fixed, void), preconditioner, CONFIG)
+    assert one["converged"] and graph["converged"]
+    assert one["launches"] < graph["launches"]
+    peak = np.max(np.abs(graph["solution"]))
+    assert np.max(np.abs(one["solution"] - graph["solution"])) <= 1e-7 * peak
+
+
+@pytest.mark.parametrize("preconditioner", ["jacobi", "two-level"])
+@pytest.mark.parametrize("slabs, rows, cols, fixed, void", [(2, 9, 130, True, False), (5, 37, 44, False, True),
+                                                            (8, 128, 128, False, False)])
+def test_attainable_residual(ns_local, preconditioner, slabs, rows, cols, fixed, void):
+    """One inner solve run far past FP32: what its correction leaves in FP64."""
+
+    config = MPIRConfig(inner_relative_tolerance=1e-9, max_outer_iterations=2, max_inner_iterations=4000)
+    one, graph = _both(ns_local, _board(ns_local, slabs, rows, cols, fixed, void), preconditioner, config)
+    assert one["history"][1][1] <= 2.0 * graph["history"][1][1]
+
+
+@pytest.mark.parametrize("preconditioner", ["jacobi", "two-level"])
+@pytest.mark.parametrize("limit", [1, 7, 540])
+def test_iteration_limit(ns_local, preconditioner, limit):
+    """Stops at the limit with the last step still owed, and across launches
+    (540 iterations are more than one launch runs; the inner tolerance is out
+    of FP32's reach)."""
+
+    config = MPIRConfig(inner_relative_tolerance=1e-30, max_outer_iterations=1, max_inner_iterations=limit)
+    one, graph = _both(ns_local, _board(ns_local, 6, 60, 70, True, False), preconditioner, config)
+    assert [h[2] for h in one["history"]] == [h[2] for h in graph["history"]] == [limit]
+    assert one["low_operator_applications"] == graph["low_operator_applications"]
+    if limit < 540:  # before the two roundings of the recurrence drift apart
+        peak = np.max(np.abs(graph["solution"]))
+        assert np.max(np.abs(one["solution"] - graph["solution"])) <= 1e-4 * peak
+
+
+def test_same_bits_every_time(ns_local):
+    problem = workloads.board_c1(3, None, 70, 61)
+    op = ns_local.MatrixFreeThermalOperator(problem, preconditioner="two-level")
+    try:
+        rhs = op.build_rhs(op.default_reference_temperature())
+        first, second = (op.device_system.solve_mpir(rhs, CONFIG) for _ in range(2))
+    finally:
+        op.close()
+    np.testing.assert_array_equal(first["solution"], second["solution"])
+    assert first["history"] == second["history"]
+
+
+def test_a_wait_that_runs_out_is_reported(ns_local):
+    op = ns_local.MatrixFreeThermalOperator(workloads.board_c1(0, None, 40, 48), preconditioner="two-level")
+    try:
+        system = op.device_system
+        rhs = op.build_rhs(op.default_reference_temperature())
+        before = system.solve_mpir(rhs, CONFIG)
+        system.set_stage_test(64)  # block 0 posts nothing
+        with pytest.raises(TimeoutError):
+            system.solve_mpir(rhs, CONFIG)
+        system.set_stage_test(0)
+        after = system.solve_mpir(rhs, CONFIG)
+    finally:
+        op.close()
+    np.testing.assert_array_equal(before["solution"], after["solution"])
