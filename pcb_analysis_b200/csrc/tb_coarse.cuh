@@ -191,58 +191,66 @@ __global__ void gj_update(double* __restrict__ A, const double* __restrict__ rk,
 // ---- blocked Gauss-Jordan inversion (no pivoting; the matrix is SPD).
 // With A split in kGjB x kGjB blocks, block step K is
 //     P = A_KK^-1,  A_KJ <- P A_KJ,  A_IJ <- A_IJ - A_IK A_KJ,  A_IK <- -A_IK P,  A_KK <- P
-// (I, J != K); after every step A holds A^-1.  Four launches per block step:
-// the diagonal block (one block of threads, unblocked elimination in shared
-// memory, pivots checked), the row panel, the trailing update (64 x 64
-// tiles, 4 x 4 outputs per thread) and the column panel.
+// (I, J != K); after every step A holds A^-1.  Three launches per block step:
+// the row panel, the trailing update (64 x 64 tiles, 4 x 4 outputs per thread)
+// and the column panel.  The diagonal block of the next step (one block of
+// threads, unblocked elimination, pivots checked) is inverted by the trailing
+// update's first block, whose tile it is, while the others work on theirs; the
+// first step's by a launch of its own.  A 2025-unknown grid: 8.4 ms with the
+// diagonal block as a fourth launch of 157 us and a trailing update of 73 us,
+// 3.6 ms now, the same bits.
 constexpr int kGjB = 64;
 constexpr int kGjLd = kGjB + 1;  // padded shared-memory row
 
-__global__ void __launch_bounds__(256) gjb_diag(double* __restrict__ A, int nc, int K, int* err) {
+// The diagonal block is the set-up's serial chain (64 dependent pivots per
+// block step, one block of threads).  A thread holds 16 entries of one row in
+// registers, columns 4 jj + jq, so that the pivot column's entry has a fixed
+// register; the pivot row and column go through shared memory in two
+// alternating buffers, one barrier per pivot: 69 us per block step (157 with the
+// block in shared memory, three barriers and one thread's reciprocal per
+// pivot).
+__device__ __forceinline__ void gjb_diag_block(double* A, int nc, int K, int* err) {
     static_assert(kGjB == 64, "256 threads: a row and 16 columns each");
-    __shared__ double D[kGjB * kGjLd];
-    __shared__ double rowk[kGjB], colk[kGjB];
-    __shared__ double s_p;
+    __shared__ double rowk[2][kGjB], colk[2][kGjB];
     const int k0 = K * kGjB;
     const int b = min(kGjB, nc - k0);
-    const int i = threadIdx.x >> 2, j0 = (threadIdx.x & 3) * 16;  // row i, columns j0 .. j0+15 of the block
-    if (i < b) {
-        for (int jj = 0; jj < 16; ++jj)
-            if (j0 + jj < b) D[i * kGjLd + j0 + jj] = A[(long long)(k0 + i) * nc + k0 + j0 + jj];
-    }
-    __syncthreads();
-    for (int k = 0; k < b; ++k) {
-        if (threadIdx.x < b) {
-            rowk[threadIdx.x] = D[k * kGjLd + threadIdx.x];
-            colk[threadIdx.x] = D[threadIdx.x * kGjLd + k];
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {  // one reciprocal per step, shared
-            const double piv = colk[k];
-            if (!(piv > 0.0) || !isfinite(piv)) atomicOr(err, 1);
-            s_p = 1.0 / piv;
-        }
-        __syncthreads();
-        const double p = s_p;
-        if (i < b) {
-            const double ci = colk[i];
+    const int i = threadIdx.x >> 2, jq = threadIdx.x & 3;
+    double* const row = A + (long long)(k0 + min(i, b - 1)) * nc + k0;
+    double D[16];
+#pragma unroll
+    for (int jj = 0; jj < 16; ++jj) D[jj] = (i < b && 4 * jj + jq < b) ? row[4 * jj + jq] : 0.0;
+#pragma unroll
+    for (int kk = 0; kk < 16; ++kk) {
+        for (int m = 0; m < 4; ++m) {
+            const int k = 4 * kk + m, buf = m & 1;
+            if (k >= b) break;  // uniform
+            if (jq == m) colk[buf][i] = D[kk];
+            if (i == k) {
+#pragma unroll
+                for (int jj = 0; jj < 16; ++jj) rowk[buf][4 * jj + jq] = D[jj];
+            }
+            __syncthreads();
+            const double piv = colk[buf][k], ci = colk[buf][i];
+            if (threadIdx.x == 0 && (!(piv > 0.0) || !isfinite(piv))) atomicOr(err, 1);
+            const double p = 1.0 / piv;
+#pragma unroll
             for (int jj = 0; jj < 16; ++jj) {
-                const int j = j0 + jj;
-                if (j >= b) break;
-                double v;
-                if (i == k && j == k) v = p;
-                else if (i == k) v = rowk[j] * p;
-                else if (j == k) v = -ci * p;
-                else v = D[i * kGjLd + j] - ci * (rowk[j] * p);
-                D[i * kGjLd + j] = v;
+                const double rp = rowk[buf][4 * jj + jq] * p;
+                const bool at = jj == kk && jq == m;  // column k
+                if (i == k) D[jj] = at ? p : rp;
+                else D[jj] = at ? -ci * p : D[jj] - ci * rp;
             }
         }
-        __syncthreads();
     }
     if (i < b) {
+#pragma unroll
         for (int jj = 0; jj < 16; ++jj)
-            if (j0 + jj < b) A[(long long)(k0 + i) * nc + k0 + j0 + jj] = D[i * kGjLd + j0 + jj];
+            if (4 * jj + jq < b) row[4 * jj + jq] = D[jj];
     }
+}
+
+__global__ void __launch_bounds__(256) gjb_diag(double* __restrict__ A, int nc, int K, int* err) {
+    gjb_diag_block(A, nc, K, err);
 }
 
 // Load the b_r x b_c block with corner (r0, c0) into shared memory (zero pad).
@@ -255,6 +263,10 @@ __device__ __forceinline__ void gjb_load(double* __restrict__ dst, const double*
 }
 
 // out (64 x 64 tile, 4 x 4 per thread) = X Y of two shared 64 x 64 blocks.
+// Rows ty + 16 a, columns tx + 16 c: the lanes of a warp read 16 successive
+// columns of Y and two rows of X, one shared-memory wavefront per load (four
+// successive columns a lane met four-way conflicts: 73 us for the trailing
+// update of a 2025-unknown grid, now 57).
 __device__ __forceinline__ void gjb_product(const double* __restrict__ X, const double* __restrict__ Y,
                                             double (&acc)[4][4]) {
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
@@ -265,9 +277,9 @@ __device__ __forceinline__ void gjb_product(const double* __restrict__ X, const 
     for (int k = 0; k < kGjB; ++k) {
         double xv[4], yv[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) xv[a] = X[(ty * 4 + a) * kGjLd + k];
+        for (int a = 0; a < 4; ++a) xv[a] = X[(ty + 16 * a) * kGjLd + k];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) yv[c] = Y[k * kGjLd + tx * 4 + c];
+        for (int c = 0; c < 4; ++c) yv[c] = Y[k * kGjLd + tx + 16 * c];
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
@@ -294,15 +306,20 @@ __global__ void __launch_bounds__(256) gjb_row(double* __restrict__ A, int nc, i
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const int i = ty * 4 + a, j = tx * 4 + c;
+            const int i = ty + 16 * a, j = tx + 16 * c;
             if (i < bk && j < bj) A[(long long)(k0 + i) * nc + j0 + j] = acc[a][c];
         }
 }
 
-// Trailing update: A_IJ -= A_IK A_KJ for I, J != K (grid = blocks x blocks).
-__global__ void __launch_bounds__(256) gjb_trailing(double* __restrict__ A, int nc, int K) {
+// Trailing update: A_IJ -= A_IK A_KJ for I, J != K (grid = blocks x blocks),
+// then A_NN <- A_NN^-1 for N = K + 1.  Block (0, 0) takes tile (N, N), so that
+// the inversion starts first, and block (N, N) tile (0, 0).
+__global__ void __launch_bounds__(256) gjb_trailing(double* A, int nc, int K, int* err) {
     extern __shared__ double sm[];
-    const int I = blockIdx.y, J = blockIdx.x;
+    const int N = K + 1;
+    const bool has_next = N * kGjB < nc;
+    int I = blockIdx.y, J = blockIdx.x;
+    if (has_next && I == J && (I == 0 || I == N)) I = J = (I == 0) ? N : 0;
     if (I == K || J == K) return;
     double* const L = sm;
     double* const U = sm + kGjB * kGjLd;
@@ -318,12 +335,16 @@ __global__ void __launch_bounds__(256) gjb_trailing(double* __restrict__ A, int 
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const int i = ty * 4 + a, j = tx * 4 + c;
+            const int i = ty + 16 * a, j = tx + 16 * c;
             if (i < bi && j < bj) {
                 double* const dst = A + (long long)(i0 + i) * nc + j0 + j;
                 *dst = *dst - acc[a][c];
             }
         }
+    if (has_next && I == N && J == N) {
+        __syncthreads();  // the tile is written
+        gjb_diag_block(A, nc, N, err);
+    }
 }
 
 // Column panel: A_IK <- -A_IK P for every row block I != K (grid.x = blocks).
@@ -345,7 +366,7 @@ __global__ void __launch_bounds__(256) gjb_col(double* __restrict__ A, int nc, i
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const int i = ty * 4 + a, j = tx * 4 + c;
+            const int i = ty + 16 * a, j = tx + 16 * c;
             if (i < bi && j < bk) A[(long long)(i0 + i) * nc + k0 + j] = -acc[a][c];
         }
 }
@@ -359,11 +380,11 @@ inline cudaError_t gauss_jordan_invert(double* A, int nc, int* err, cudaStream_t
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gjb_col, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const int nb = (nc + kGjB - 1) / kGjB;
+    gjb_diag<<<1, 256, 0, stream>>>(A, nc, 0, err);
     for (int K = 0; K < nb; ++K) {
-        gjb_diag<<<1, 256, 0, stream>>>(A, nc, K, err);
         if (nb > 1) {
             gjb_row<<<nb, 256, smem, stream>>>(A, nc, K);
-            gjb_trailing<<<dim3(nb, nb), 256, smem, stream>>>(A, nc, K);
+            gjb_trailing<<<dim3(nb, nb), 256, smem, stream>>>(A, nc, K, err);
             gjb_col<<<nb, 256, smem, stream>>>(A, nc, K);
         }
     }

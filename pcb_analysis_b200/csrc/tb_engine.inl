@@ -728,7 +728,7 @@ int engine_submit(tb_engine* e, const tb_system_desc* d, const double* rhs, cons
         coarse_work = nullptr;
         TB_ENGINE_CUDA(cudaMemsetAsync(x64, 0, sizeof(double) * L.L, e->io));
         TB_ENGINE_CUDA(cudaMemsetAsync(r64, 0, sizeof(double) * L.L, e->io));
-        e->kernel_launches += 2 + 4 * 27 + 2 + 4LL * ((nc + kGjB - 1) / kGjB);
+        e->kernel_launches += 2 + 4 * 27 + 2 + 1 + 3LL * ((nc + kGjB - 1) / kGjB);
     }
     if (x0) {
         pack_nodes<double, double><<<nb, kVecThreads, 0, e->io>>>(x64, st_x0, L);

@@ -488,7 +488,7 @@ int build_multilevel(tb_system* s) {
     if (rc == TB_OK) {
         const int mb = grid_for(nn, kVecThreads, sb);
         coarse_symmetrize<<<mb, kVecThreads, 0, st>>>(work, s->coarse_inv64, s->coarse_inv32, cl.nc, cl.ld);
-        s->kernel_launches += 1 + 4LL * ml_cdiv(cl.nc, kGjB);
+        s->kernel_launches += 1 + 3LL * ml_cdiv(cl.nc, kGjB) + 1;
         check_launch();
     }
     int err = 0;

@@ -1603,7 +1603,7 @@ int build_coarse(tb_system* s, int block) {
         if (rc == TB_OK && gauss_jordan_invert(work, cl.nc, s->d_err, st) != cudaSuccess)
             rc = fail(TB_ECUDA, "coarse inversion launch failed");
         coarse_symmetrize<<<mb, kVecThreads, 0, st>>>(work, s->coarse_inv64, s->coarse_inv32, cl.nc, cl.ld);
-        s->kernel_launches += 2 + 4LL * cdiv(cl.nc, kGjB);
+        s->kernel_launches += 2 + 3LL * cdiv(cl.nc, kGjB) + 1;
         check_launch();
     }
     int err = 0;
