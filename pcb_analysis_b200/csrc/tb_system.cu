@@ -980,11 +980,12 @@ std::vector<ApplyPlan> plan_candidates(const Layout& L, unsigned long long speci
                 p.kind = kind;
                 p.rows = rows;
                 p.tma = tma;
+                // Not the deeper pipeline (kDeepStages, open to
+                // tb_set_apply_plan): alone it is as fast (294.0 against 294.9
+                // us on c3), but its blocks take 185 KB of an SM's shared
+                // memory, which leaves the kernel behind it a small L1: the
+                // fine pass 382 against 349 us, an iteration 1248 against 1214.
                 out.push_back(p);
-                if (kind == 0 && tma == 1 && rows <= 16) {  // the deeper tensor-copy pipeline
-                    p.stages = kDeepStages;
-                    out.push_back(p);
-                }
             }
         }
     }
