@@ -37,7 +37,10 @@
 namespace tb {
 
 constexpr int kBatchMax = 256;                     // boards in one schedule
-constexpr int kBatchChunkQuads = kVecThreads * 8;  // 2048 quads = 8192 nodes per vector chunk
+// 1024 quads = 4096 nodes per vector chunk: ten boards of 27 .. 590 thousand
+// nodes then fill the device (580 chunks; 290 of twice the size left an SM two
+// blocks: update 20.2 us against 15.6 here).
+constexpr int kBatchChunkQuads = kVecThreads * 4;
 constexpr int kBatchHist = 64;                     // outer steps recorded per board
 
 enum BatchPhase {
@@ -112,7 +115,10 @@ struct BatchSchedule {
 };
 
 enum { ITEMS_TILE32 = 0, ITEMS_TILE64 = 1, ITEMS_CHUNK = 2, ITEMS_PATCH = 3, ITEMS_CROW = 4 };
-constexpr int kCoarseRows = 8;  // rows of the coarse inverse per item (one warp each)
+// Rows of the coarse inverse per item, four a warp: an item stages R, takes a
+// ticket and merges its part of R.c, some 4 us beside 1 us per row of reading
+// (ten boards of 2,000 unknowns: 53 us with eight rows, one a warp, 47).
+constexpr int kCoarseRows = 32;
 
 __global__ void batch_set_schedule(BatchSchedule value, BatchSchedule* dst) {
     const int* src = reinterpret_cast<const int*>(&value);
@@ -139,11 +145,13 @@ __global__ void batch_release(BatchStatus* status) {
     if (threadIdx.x == 0 && blockIdx.x == 0) status->phase = PH_IDLE;
 }
 
-// The schedule's slots and one prefix array in shared memory.
+// The schedule's slots and one prefix array in shared memory, and per board
+// whether (how) the kernel is to work on it.
 struct ItemMap {
     int n;
     int slot[kBatchMax];
     int prefix[kBatchMax + 1];
+    unsigned char go[kBatchMax];
 };
 
 template <int WHICH>
@@ -176,12 +184,36 @@ __device__ __forceinline__ int find_board(const ItemMap& m, int t) {
 __device__ __forceinline__ int load_phase(const BatchStatus* s) { return *reinterpret_cast<const volatile int*>(&s->phase); }
 __device__ __forceinline__ int load_state(const SolveCtl* c) { return *reinterpret_cast<const volatile int*>(&c->state); }
 
-// Board ticket: true in every thread of the block that finished the board's
-// last item.  Thread 0 must have stored the block's partial before the call.
-__device__ __forceinline__ bool last_item(unsigned int* counter, int items, bool* flag) {
-    __threadfence();
+// Start of a batched kernel of an iteration: the items (the schedule stands
+// still while a chunk runs, so they are read ahead of the dependency wait),
+// then every board's `select` at once.  What it looks at (phase, solve state)
+// is changed by the kernel itself only after the board's last item.
+template <int WHICH, class Select>
+__device__ __forceinline__ void enter_items(const BatchInstance* __restrict__ table,
+                                            const BatchSchedule* __restrict__ sched, ItemMap& m, Select select) {
+    load_items<WHICH>(sched, m);
+    pdl_enter();
+    for (int k = threadIdx.x; k < m.n; k += blockDim.x) m.go[k] = (unsigned char)select(table + m.slot[k]);
     __syncthreads();
-    if (threadIdx.x == 0) *flag = (atomicAdd(counter, 1u) == (unsigned)(items - 1));
+}
+// A board whose inner PCG runs, and (two-level) one about to take its first
+// coarse step.
+__device__ __forceinline__ int board_running(const BatchInstance* I) {
+    return load_phase(I->status) == PH_INNER && load_state(I->ctl) == ST_RUNNING ? 1 : 0;
+}
+__device__ __forceinline__ int board_running_or_starting(const BatchInstance* I) {
+    return load_phase(I->status) == PH_PRECOND ? 2 : board_running(I);
+}
+
+// Board ticket: true in every thread of the block that finished the board's
+// last item.  Thread 0 must have stored the block's partial before the call;
+// only its writes are published (the other threads' are read by later kernels).
+__device__ __forceinline__ bool last_item(unsigned int* counter, int items, bool* flag) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        *flag = (atomicAdd(counter, 1u) == (unsigned)(items - 1));
+    }
     __syncthreads();
     const bool last = *flag;
     if (last) __threadfence();
@@ -212,12 +244,11 @@ __global__ void __launch_bounds__(16 * ROWS, ApplyOccupancy<float, ROWS>::min_bl
     __shared__ ItemMap m;
     __shared__ __align__(16) unsigned char p_raw[sizeof(ApplyParams<float>)];
     __shared__ __align__(16) unsigned char red_raw[sizeof(Acc32) * 32];
-    __shared__ int s_go;
     __shared__ bool s_last;
     ApplyParams<float>* const sP = reinterpret_cast<ApplyParams<float>*>(p_raw);
     Acc32* const red = reinterpret_cast<Acc32*>(red_raw);
     __shared__ int s_t;
-    load_items<ITEMS_TILE32>(sched, m);
+    enter_items<ITEMS_TILE32>(table, sched, m, board_running);
     const int total = m.prefix[m.n];
     unsigned int* const grab = const_cast<unsigned int*>(sched->grab);
     int seq = 0;
@@ -233,13 +264,12 @@ __global__ void __launch_bounds__(16 * ROWS, ApplyOccupancy<float, ROWS>::min_bl
         if (t >= total) break;
         const int k = find_board(m, t);
         const BatchInstance* I = table + m.slot[k];
-        if (threadIdx.x == 0) s_go = load_phase(I->status) == PH_INNER && load_state(I->ctl) == ST_RUNNING;
-        copy_params(sP, &I->a32);
-        __syncthreads();
-        if (!s_go) {
-            __syncthreads();
+        if (!m.go[k]) {
+            __syncthreads();  // s_t has been read
             continue;
         }
+        copy_params(sP, &I->a32);
+        __syncthreads();
         const int lt = t - m.prefix[k];
         const int gx = I->gx32;
         float dot = 0.f;
@@ -368,8 +398,7 @@ __global__ void __launch_bounds__(16 * ROWS, 1)
 }
 
 // ------------------------------------------------------------ vector chunks
-// Walks the chunks of the boards that `select` accepts (decided by thread 0
-// of the block, shared with the block).  `body(I, q0, q1, acc)` works on quads
+// Walks the chunks of the boards that `select` accepts.  `body(I, q0, q1, acc)` works on quads
 // [q0, q1) of the board; with NA > 0 its accumulators are reduced per board
 // and `finish(I, tot)` runs in thread 0 of the board's last chunk.
 template <int NA, class Select, class Body, class Finish>
@@ -378,19 +407,14 @@ __device__ __forceinline__ void batch_chunks(const BatchInstance* __restrict__ t
                                              Select select, Body body, Finish finish) {
     __shared__ ItemMap m;
     __shared__ __align__(16) unsigned char red_raw[sizeof(Acc32) * (NA > 0 ? NA : 1) * 32];
-    __shared__ int s_go;
     __shared__ bool s_last;
     Acc32* const red = reinterpret_cast<Acc32*>(red_raw);
-    load_items<ITEMS_CHUNK>(sched, m);
+    enter_items<ITEMS_CHUNK>(table, sched, m, select);
     const int total = m.prefix[m.n];
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
         const int k = find_board(m, t);
         const BatchInstance* I = table + m.slot[k];
-        if (threadIdx.x == 0) s_go = select(I);
-        __syncthreads();
-        const bool go = s_go;
-        __syncthreads();
-        if (!go) continue;
+        if (!m.go[k]) continue;
         const int lc = t - m.prefix[k];
         const long long q0 = (long long)lc * kBatchChunkQuads;
         const long long q1 = min(q0 + kBatchChunkQuads, I->nq);
@@ -427,7 +451,7 @@ __global__ void __launch_bounds__(kVecThreads)
     batch_update32(const BatchInstance* __restrict__ table, const BatchSchedule* __restrict__ sched) {
     batch_chunks<2>(
         table, sched, 1,
-        [](const BatchInstance* I) { return load_phase(I->status) == PH_INNER && load_state(I->ctl) == ST_RUNNING; },
+        board_running,
         [](const BatchInstance* I, long long q0, long long q1, Acc32 (&acc)[2]) {
             // the step x += alpha p is taken by the direction kernel (or the
             // outer finish), as in the single-board PCG
@@ -474,20 +498,13 @@ __device__ __forceinline__ void x_step(float4* __restrict__ x, const float4 pv, 
 __global__ void __launch_bounds__(kVecThreads)
     batch_direction32(const BatchInstance* __restrict__ table, const BatchSchedule* __restrict__ sched) {
     __shared__ ItemMap m;
-    __shared__ int s_go;
     __shared__ bool s_last;
-    load_items<ITEMS_CHUNK>(sched, m);
+    enter_items<ITEMS_CHUNK>(table, sched, m, board_running_or_starting);
     const int total = m.prefix[m.n];
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
         const int k = find_board(m, t);
         const BatchInstance* I = table + m.slot[k];
-        if (threadIdx.x == 0) {
-            const int ph = load_phase(I->status);
-            s_go = (ph == PH_INNER && load_state(I->ctl) == ST_RUNNING) ? 1 : (ph == PH_PRECOND ? 2 : 0);
-        }
-        __syncthreads();
-        const int go = s_go;
-        __syncthreads();
+        const int go = m.go[k];
         if (!go) continue;
         const long long q0 = (long long)(t - m.prefix[k]) * kBatchChunkQuads;
         const long long q1 = min(q0 + kBatchChunkQuads, I->nq);
@@ -557,20 +574,14 @@ __global__ void __launch_bounds__(kVecThreads)
 __global__ void __launch_bounds__(256)
     batch_restrict(const BatchInstance* __restrict__ table, const BatchSchedule* __restrict__ sched) {
     __shared__ ItemMap m;
-    load_items<ITEMS_PATCH>(sched, m);
+    enter_items<ITEMS_PATCH>(table, sched, m, board_running_or_starting);
     const int total = m.prefix[m.n];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
     for (int t = blockIdx.x * wpb + warp; t < total; t += gridDim.x * wpb) {
         const int k = find_board(m, t);
         const BatchInstance* I = table + m.slot[k];
-        int go = 0;
-        if (lane == 0) {
-            const int ph = load_phase(I->status);
-            go = ((ph == PH_INNER && load_state(I->ctl) == ST_RUNNING) || ph == PH_PRECOND) ? 1 : 0;
-        }
-        go = __shfl_sync(0xffffffffu, go, 0);
-        if (!go) continue;
+        if (!m.go[k]) continue;
         const CoarseLayout cl = I->cl;
         const Layout lay = I->lay;
         const int P = t - m.prefix[k];
@@ -608,11 +619,10 @@ __global__ void __launch_bounds__(256)
     extern __shared__ float s_rc[];
     __shared__ ItemMap m;
     __shared__ __align__(16) unsigned char red_raw[sizeof(Acc32) * 32];
-    __shared__ int s_go;
     __shared__ bool s_last;
     Acc32* const red = reinterpret_cast<Acc32*>(red_raw);
     __shared__ int s_t;
-    load_items<ITEMS_CROW>(sched, m);
+    enter_items<ITEMS_CROW>(table, sched, m, board_running_or_starting);
     const int total = m.prefix[m.n];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned int* const grab = const_cast<unsigned int*>(sched->grab) + 2;
@@ -625,22 +635,18 @@ __global__ void __launch_bounds__(256)
         if (t >= total) break;
         const int k = find_board(m, t);
         const BatchInstance* I = table + m.slot[k];
-        if (threadIdx.x == 0) {
-            const int ph = load_phase(I->status);
-            s_go = (ph == PH_INNER && load_state(I->ctl) == ST_RUNNING) ? 1 : (ph == PH_PRECOND ? 2 : 0);
-        }
-        __syncthreads();
-        const int go = s_go;
+        const int go = m.go[k];
         if (!go) {
-            __syncthreads();
+            __syncthreads();  // s_t has been read
             continue;
         }
         const int nc = I->cl.nc, ld = I->cl.ld;
         for (int i = threadIdx.x; i < ld; i += blockDim.x) s_rc[i] = I->rc[i];
         __syncthreads();
-        const int row = (t - m.prefix[k]) * kCoarseRows + warp;
         Acc32 acc[1];
-        if (warp < kCoarseRows && row < nc) {
+        for (int u = warp; u < kCoarseRows; u += blockDim.x >> 5) {
+            const int row = (t - m.prefix[k]) * kCoarseRows + u;
+            if (row >= nc) break;
             const float sum = coarse_row(I->minv + (long long)row * ld, s_rc, ld, lane);
             if (lane == 0) {
                 I->cvec[row] = sum;

@@ -107,19 +107,21 @@ int engine_grid32(tb_engine* e) {
     return TB_OK;
 }
 
+// The kernels of an iteration are chained by programmatic dependent launch:
+// each reads the schedule and waits for its predecessor only then.
+using BatchKernel = void (*)(const BatchInstance*, const BatchSchedule*);
+int engine_launch(tb_engine* e, BatchKernel kernel, int grid, int threads, size_t smem) {
+    return launch_pdl(kernel, dim3(grid), dim3(threads), smem, e->stream, (const BatchInstance*)e->d_table,
+                      (const BatchSchedule*)e->d_sched) == cudaSuccess
+               ? TB_OK
+               : TB_ECUDA;
+}
+
 int engine_launch_apply32(tb_engine* e) {
-    const dim3 grid(e->grid32), block(16 * e->rows32);
-    const size_t sm = e->smem32;
-    if (e->tma32) {
-        if (e->rows32 == 8) batch_apply32<8, true><<<grid, block, sm, e->stream>>>(e->d_table, e->d_sched);
-        else if (e->rows32 == 16) batch_apply32<16, true><<<grid, block, sm, e->stream>>>(e->d_table, e->d_sched);
-        else batch_apply32<32, true><<<grid, block, sm, e->stream>>>(e->d_table, e->d_sched);
-    } else {
-        if (e->rows32 == 8) batch_apply32<8><<<grid, block, sm, e->stream>>>(e->d_table, e->d_sched);
-        else if (e->rows32 == 16) batch_apply32<16><<<grid, block, sm, e->stream>>>(e->d_table, e->d_sched);
-        else batch_apply32<32><<<grid, block, sm, e->stream>>>(e->d_table, e->d_sched);
-    }
-    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ECUDA;
+    BatchKernel kernel;
+    if (e->tma32) kernel = e->rows32 == 8 ? batch_apply32<8, true> : (e->rows32 == 16 ? batch_apply32<16, true> : batch_apply32<32, true>);
+    else kernel = e->rows32 == 8 ? batch_apply32<8> : (e->rows32 == 16 ? batch_apply32<16> : batch_apply32<32>);
+    return engine_launch(e, kernel, e->grid32, 16 * e->rows32, e->smem32);
 }
 
 int engine_capture(tb_engine* e) {
@@ -136,13 +138,10 @@ int engine_capture(tb_engine* e) {
     for (int i = 0; i < kChunk && rc == TB_OK; ++i) {
         rc = engine_launch_apply32(e);
         if (rc != TB_OK) break;
-        batch_update32<<<e->gridv, kVecThreads, 0, e->stream>>>(e->d_table, e->d_sched);
-        if (e->precond) {
-            batch_restrict<<<e->gridr, 256, 0, e->stream>>>(e->d_table, e->d_sched);
-            batch_coarse<<<e->gridc, 256, sizeof(float) * 2048, e->stream>>>(e->d_table, e->d_sched);
-        }
-        batch_direction32<<<e->gridv, kVecThreads, 0, e->stream>>>(e->d_table, e->d_sched);
-        if (cudaGetLastError() != cudaSuccess) rc = TB_ECUDA;
+        rc = engine_launch(e, batch_update32, e->gridv, kVecThreads, 0);
+        if (rc == TB_OK && e->precond) rc = engine_launch(e, batch_restrict, e->gridr, 256, 0);
+        if (rc == TB_OK && e->precond) rc = engine_launch(e, batch_coarse, e->gridc, 256, sizeof(float) * 2048);
+        if (rc == TB_OK) rc = engine_launch(e, batch_direction32, e->gridv, kVecThreads, 0);
     }
     const cudaError_t end = cudaStreamEndCapture(e->stream, &graph);
     if (rc != TB_OK || end != cudaSuccess) {
