@@ -141,6 +141,7 @@ struct tb_system {
     unsigned int* counter = nullptr;
     SolveCtl* ctl = nullptr;
     SolveCtl* h_ctl = nullptr;  // pinned, 2 slots
+    int* h_err = nullptr;       // pinned copy of *stage_err, behind them
     KernelClock* clocks = nullptr;  // [0] FP32 apply (p.Ap), [1] FP64 apply (residual / PCG), [2] multilevel fine pass
     // graphs: two chunk slots per precision, kept in flight alternately
     ChunkSlot slots32[2], slots64[2];
@@ -1143,10 +1144,9 @@ int encode_apply_maps(tb_system* s) {
 // A block of the tensor-copy staging that gave up waiting for its tiles set
 // the error word: the action is incomplete.
 int check_stage(tb_system* s) {
-    int err = 0;
-    TB_CUDA(cudaMemcpyAsync(&err, s->stage_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    TB_CUDA(cudaMemcpyAsync(s->h_err, s->stage_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     TB_CUDA(cudaStreamSynchronize(s->stream));
-    if (err != 0) {
+    if (*s->h_err != 0) {
         TB_CUDA(cudaMemsetAsync(s->stage_err, 0, sizeof(int), s->stream));
         return fail(TB_ETIMEOUT, "a block of the operator or of the staged fine pass gave up waiting for its staged tiles");
     }
@@ -1223,9 +1223,10 @@ int begin_system(int slabs, int rows, int cols, const double* thick, const doubl
     TB_CHECK(alloc_n(s, &s->clocks, 3));
     {
         void* h = nullptr;
-        TB_CUDA(cudaMallocHost(&h, 2 * sizeof(SolveCtl)));
+        TB_CUDA(cudaMallocHost(&h, 2 * sizeof(SolveCtl) + sizeof(int)));
         s->h_ctl = static_cast<SolveCtl*>(h);
-        std::memset(s->h_ctl, 0, 2 * sizeof(SolveCtl));
+        std::memset(h, 0, 2 * sizeof(SolveCtl) + sizeof(int));
+        s->h_err = reinterpret_cast<int*>(s->h_ctl + 2);
     }
     TB_CUDA(cudaMemsetAsync(s->counter, 0, sizeof(unsigned int), s->stream));
     TB_CUDA(cudaMemsetAsync(s->ctl, 0, sizeof(SolveCtl), s->stream));
@@ -1338,35 +1339,45 @@ void destroy_impl(tb_system* s) {
     delete s;
 }
 
+// Blocks of pack_nodes and unpack_nodes: a warp per node row, at most 16 blocks an SM.
+int pack_grid(const Layout& L, int sms) {
+    return grid_for((long long)(L.S + 1) * (L.R + 1), kPackThreads / 32, sms * 16);
+}
+
 // Copy a flat host or device node array into a padded device field.
 template <typename T>
 int load_nodes(tb_system* s, T* dst, const T* src, bool src_on_device) {
     const Layout& L = s->lay;
-    const int nb = grid_for(L.L, kVecThreads, 148 * 16);
+    const int nb = pack_grid(L, s->sms);
     const T* flat = src;
     if (!src_on_device) {
         TB_CHECK(ensure_stage(s, sizeof(T) * (size_t)L.N));
         TB_CHECK(host_to_device(s, s->stage, src, sizeof(T) * L.N));
         flat = static_cast<const T*>(s->stage);
     }
-    pack_nodes<T, T><<<nb, kVecThreads, 0, s->stream>>>(dst, flat, L);
+    pack_nodes<T, T><<<nb, kPackThreads, 0, s->stream>>>(dst, flat, L);
     TB_CUDA(cudaGetLastError());
     s->kernel_launches += 1;
     return TB_OK;
 }
 
+// `pdl`: launched as a programmatic dependent of the kernel that wrote `src`.
 template <typename T>
-int store_nodes(tb_system* s, T* dst, const T* src, bool dst_on_device) {
+int store_nodes(tb_system* s, T* dst, const T* src, bool dst_on_device, bool pdl = false) {
     const Layout& L = s->lay;
-    const int nb = grid_for(L.N, kVecThreads, 148 * 16);
+    const int nb = pack_grid(L, s->sms);
     if (dst_on_device) {
-        unpack_nodes<T, T><<<nb, kVecThreads, 0, s->stream>>>(dst, src, L);
-        TB_CUDA(cudaGetLastError());
+        if (pdl) {
+            TB_CUDA(launch_pdl(unpack_nodes<T, T>, dim3(nb), dim3(kPackThreads), 0, s->stream, dst, src, L));
+        } else {
+            unpack_nodes<T, T><<<nb, kPackThreads, 0, s->stream>>>(dst, src, L);
+            TB_CUDA(cudaGetLastError());
+        }
         s->kernel_launches += 1;
         return TB_OK;
     }
     TB_CHECK(ensure_stage(s, sizeof(T) * (size_t)L.N));
-    unpack_nodes<T, T><<<nb, kVecThreads, 0, s->stream>>>(static_cast<T*>(s->stage), src, L);
+    unpack_nodes<T, T><<<nb, kPackThreads, 0, s->stream>>>(static_cast<T*>(s->stage), src, L);
     TB_CUDA(cudaGetLastError());
     s->kernel_launches += 1;
     TB_CHECK(device_to_host(s, dst, s->stage, sizeof(T) * L.N));
@@ -2466,14 +2477,19 @@ static int apply_any(tb_system* s, const void* x, void* y, bool f64, bool dev, b
         if (stiffness)
             TB_CHECK((launch_apply<double, MODE_STIFFNESS, EPI_STORE>(s, P)));
         else
-            TB_CHECK((launch_apply<double, MODE_OPERATOR, EPI_STORE>(s, P)));
-        TB_CHECK(store_nodes<double>(s, static_cast<double*>(y), s->r64, dev));
+            TB_CHECK((launch_apply<double, MODE_OPERATOR, EPI_STORE>(s, P, true)));
+        TB_CHECK(store_nodes<double>(s, static_cast<double*>(y), s->r64, dev, true));
     } else {
         TB_CHECK(load_nodes<float>(s, s->p32, static_cast<const float*>(x), dev));
         const ApplyParams<float> P = apply_params<float>(s, s->p32, s->q32, nullptr);
-        TB_CHECK((launch_apply<float, MODE_OPERATOR, EPI_STORE>(s, P)));
+        TB_CHECK((launch_apply<float, MODE_OPERATOR, EPI_STORE>(s, P, true)));
+        if (dev) {  // one wait for the three kernels and the staging's error word
+            TB_CHECK(store_nodes<float>(s, static_cast<float*>(y), s->q32, true, true));
+            s->kernel_launches += 1;
+            return check_stage(s);
+        }
         TB_CHECK(check_stage(s));
-        TB_CHECK(store_nodes<float>(s, static_cast<float*>(y), s->q32, dev));
+        TB_CHECK(store_nodes<float>(s, static_cast<float*>(y), s->q32, false));
     }
     s->kernel_launches += 1;
     if (dev) TB_CUDA(cudaStreamSynchronize(s->stream));

@@ -27,25 +27,40 @@ struct Layout {
 };
 
 // ----------------------------------------------------------------- layout
+// Flat (caller's) to padded node rows and back: a warp per node row, its lanes
+// along the row, so that no element needs a division by the row length.
+// Chained by programmatic dependent launch where the caller asks: with one
+// wait instead of three, the FP32 action on c2's 3.4 M nodes takes 54 us from
+// the caller's tensors (84 before; its two copies are 7 us each).
+constexpr int kPackThreads = 256;
 template <typename D, typename Src>
-__global__ void pack_nodes(D* __restrict__ dst, const Src* __restrict__ src, Layout lay) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const int cols = lay.C + 1;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < lay.L; i += stride) {
-        const long long line = i / lay.Xp;
-        const int x = (int)(i - line * lay.Xp);
-        dst[i] = (x < cols) ? (D)src[line * cols + x] : (D)0;
+__global__ void __launch_bounds__(kPackThreads) pack_nodes(D* __restrict__ dst, const Src* __restrict__ src, Layout lay) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int cols = lay.C + 1, lane = threadIdx.x & 31;
+    const long long lines = (long long)(lay.S + 1) * (lay.R + 1);
+    const long long stride = (long long)gridDim.x * (kPackThreads / 32);
+    for (long long line = (long long)blockIdx.x * (kPackThreads / 32) + (threadIdx.x >> 5); line < lines; line += stride) {
+        const Src* const s = src + line * cols;
+        D* const d = dst + line * lay.Xp;
+#pragma unroll 4
+        for (int x = lane; x < lay.Xp; x += 32) d[x] = (x < cols) ? (D)s[x] : (D)0;
     }
 }
 
 template <typename D, typename Src>
-__global__ void unpack_nodes(D* __restrict__ dst, const Src* __restrict__ src, Layout lay) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const int cols = lay.C + 1;
-    for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < lay.N; n += stride) {
-        const long long line = n / cols;
-        const int x = (int)(n - line * cols);
-        dst[n] = (D)src[line * lay.Xp + x];
+__global__ void __launch_bounds__(kPackThreads)
+    unpack_nodes(D* __restrict__ dst, const Src* __restrict__ src, Layout lay) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int cols = lay.C + 1, lane = threadIdx.x & 31;
+    const long long lines = (long long)(lay.S + 1) * (lay.R + 1);
+    const long long stride = (long long)gridDim.x * (kPackThreads / 32);
+    for (long long line = (long long)blockIdx.x * (kPackThreads / 32) + (threadIdx.x >> 5); line < lines; line += stride) {
+        const Src* const s = src + line * lay.Xp;
+        D* const d = dst + line * cols;
+#pragma unroll 4
+        for (int x = lane; x < cols; x += 32) d[x] = (D)s[x];
     }
 }
 
