@@ -178,7 +178,8 @@ int tb_solve_pcg_f64_ml_device(tb_system* system, const double* d_rhs, double* d
  * and each wait gives up after `polls` polls; every block then records the
  * timeout and returns with nothing in flight, and the apply or solve fails
  * with TB_ETIMEOUT.  0 restores normal staging.  Affects launch plans with
- * tensor-copy staging only (tb_set_apply_plan). */
+ * tensor-copy staging (tb_set_apply_plan), and the cooperative PCG kernel of
+ * small boards, whose first block then posts nothing. */
 int tb_set_stage_test(tb_system* system, int32_t polls);
 
 /* Launch form of the multilevel preconditioner's fine pass in the inner FP32
@@ -222,7 +223,9 @@ int tb_get_timing(const tb_system* system, double* ms4, int64_t* launches4);
  *         resident blocks that share the board's (tile, node plane) pairs
  *         evenly (same output bits as kind 0, no second partial wave).
  * Chosen at creation by timing the candidates on the board (cached per slab
- * count and board size); tb_set_apply_plan overrides the choice.
+ * count and board size); tb_set_apply_plan overrides the choice, and has the
+ * inner PCG of a small board run as graph-captured kernels with this plan
+ * instead of the one cooperative kernel it otherwise takes.
  * tb_set_tile_rows(rows) is tb_set_apply_plan({0, rows, 0, 0, 0}). */
 int tb_set_apply_plan(tb_system* system, const int32_t* plan5);
 int tb_get_apply_plan(const tb_system* system, int32_t* plan5);

@@ -865,7 +865,7 @@ int kernels_per_iteration(const tb_system* s, bool f64) {
 // Run PCG chunks until the device state leaves ST_RUNNING.  Two chunks are in
 // flight: the next one is queued before the state after the previous one is
 // read, and the kernels of a finished PCG return at once.  Those returns are
-// not free (on c3 a finished iteration's 34 launches still take about 0.18
+// not free (on c3 a finished iteration's launches, then 34, took about 0.18
 // ms), so when the residual's decay since the previous chunk says that the
 // chunk in flight will reach the tolerance with a quarter of its iterations
 // to spare, no further chunk is queued until its state has been read.  A
