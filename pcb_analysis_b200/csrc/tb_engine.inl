@@ -691,7 +691,7 @@ int engine_submit(tb_engine* e, const tb_system_desc* d, const double* rhs, cons
     build_rf<<<nb, kVecThreads, 0, e->io>>>(rf64, rf32, flags, st_robin, st_free, L);
     build_diagonal<<<nb, kVecThreads, 0, e->io>>>(st_diag, st_dinv, dinv32, st_err, kin64, kz64, rf64, st_geo,
                                                   st_geo + L.S, st_geo + L.S + L.C, L);
-    pack_nodes<double, double><<<pack_grid(L, e->sms), kPackThreads, 0, e->io>>>(b64, st_rhs, L);
+    pack_kernel<double>(pack_shape(L))<<<pack_grid(L, e->sms), kPackThreads, 0, e->io>>>(b64, st_rhs, L, pack_shape(L));
     TB_ENGINE_CUDA(cudaGetLastError());
     e->kernel_launches += 5;
     if (nc > 0) {
@@ -730,7 +730,7 @@ int engine_submit(tb_engine* e, const tb_system_desc* d, const double* rhs, cons
         e->kernel_launches += 2 + 4 * 27 + 2 + 1 + 3LL * ((nc + kGjB - 1) / kGjB);
     }
     if (x0) {
-        pack_nodes<double, double><<<pack_grid(L, e->sms), kPackThreads, 0, e->io>>>(x64, st_x0, L);
+        pack_kernel<double>(pack_shape(L))<<<pack_grid(L, e->sms), kPackThreads, 0, e->io>>>(x64, st_x0, L, pack_shape(L));
         TB_ENGINE_CUDA(cudaGetLastError());
         e->kernel_launches += 1;
     }
@@ -842,8 +842,8 @@ int engine_collect(tb_engine* e, long long ticket, double* x, tb_mpir_result* re
     if (x) {
         void* tmp = nullptr;
         TB_CUDA(cudaMallocFromPoolAsync(&tmp, sizeof(double) * (size_t)L.N, e->pool, e->io));
-        unpack_nodes<double, double>
-            <<<pack_grid(L, e->sms), kPackThreads, 0, e->io>>>(static_cast<double*>(tmp), b->inst.x64, L);
+        unpack_kernel<double>(pack_shape(L))<<<pack_grid(L, e->sms), kPackThreads, 0, e->io>>>(
+            static_cast<double*>(tmp), b->inst.x64, L, pack_shape(L));
         TB_CUDA(cudaGetLastError());
         e->kernel_launches += 1;
         TB_CUDA(cudaMemcpyAsync(x, tmp, sizeof(double) * (size_t)L.N, cudaMemcpyDeviceToHost, e->io));

@@ -1339,9 +1339,10 @@ void destroy_impl(tb_system* s) {
     delete s;
 }
 
-// Blocks of pack_nodes and unpack_nodes: a warp per node row, at most 16 blocks an SM.
+// Blocks of pack_nodes and unpack_nodes: a group of lanes per row segment, at most 16 blocks an SM.
 int pack_grid(const Layout& L, int sms) {
-    return grid_for((long long)(L.S + 1) * (L.R + 1), kPackThreads / 32, sms * 16);
+    const PackShape p = pack_shape(L);
+    return grid_for((long long)(L.S + 1) * (L.R + 1) * p.segments, kPackThreads / p.lanes, sms * 16);
 }
 
 // Copy a flat host or device node array into a padded device field.
@@ -1355,7 +1356,7 @@ int load_nodes(tb_system* s, T* dst, const T* src, bool src_on_device) {
         TB_CHECK(host_to_device(s, s->stage, src, sizeof(T) * L.N));
         flat = static_cast<const T*>(s->stage);
     }
-    pack_nodes<T, T><<<nb, kPackThreads, 0, s->stream>>>(dst, flat, L);
+    pack_kernel<T>(pack_shape(L))<<<nb, kPackThreads, 0, s->stream>>>(dst, flat, L, pack_shape(L));
     TB_CUDA(cudaGetLastError());
     s->kernel_launches += 1;
     return TB_OK;
@@ -1368,16 +1369,17 @@ int store_nodes(tb_system* s, T* dst, const T* src, bool dst_on_device, bool pdl
     const int nb = pack_grid(L, s->sms);
     if (dst_on_device) {
         if (pdl) {
-            TB_CUDA(launch_pdl(unpack_nodes<T, T>, dim3(nb), dim3(kPackThreads), 0, s->stream, dst, src, L));
+            TB_CUDA(launch_pdl(unpack_kernel<T>(pack_shape(L)), dim3(nb), dim3(kPackThreads), 0, s->stream, dst, src, L,
+                               pack_shape(L)));
         } else {
-            unpack_nodes<T, T><<<nb, kPackThreads, 0, s->stream>>>(dst, src, L);
+            unpack_kernel<T>(pack_shape(L))<<<nb, kPackThreads, 0, s->stream>>>(dst, src, L, pack_shape(L));
             TB_CUDA(cudaGetLastError());
         }
         s->kernel_launches += 1;
         return TB_OK;
     }
     TB_CHECK(ensure_stage(s, sizeof(T) * (size_t)L.N));
-    unpack_nodes<T, T><<<nb, kPackThreads, 0, s->stream>>>(static_cast<T*>(s->stage), src, L);
+    unpack_kernel<T>(pack_shape(L))<<<nb, kPackThreads, 0, s->stream>>>(static_cast<T*>(s->stage), src, L, pack_shape(L));
     TB_CUDA(cudaGetLastError());
     s->kernel_launches += 1;
     TB_CHECK(device_to_host(s, dst, s->stage, sizeof(T) * L.N));

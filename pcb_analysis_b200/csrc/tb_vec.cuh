@@ -27,41 +27,91 @@ struct Layout {
 };
 
 // ----------------------------------------------------------------- layout
-// Flat (caller's) to padded node rows and back: a warp per node row, its lanes
-// along the row, so that no element needs a division by the row length.
+// Flat (caller's) to padded node rows and back.  A group of lanes takes a
+// segment of a node row, so that no element needs a division by the row
+// length: up to kPackSegment nodes of a long row (one row is then spread over
+// several groups), a whole row otherwise, with as many lanes as it can use.
+// FP32 actions of strips, with one warp per row and now: a 1 x 100,000 x 8 board
+// (18 rows) 410 and 53 us, a 100,000 x 1 x 8 board (rows of four) 180 and 101.
 // Chained by programmatic dependent launch where the caller asks: with one
 // wait instead of three, the FP32 action on c2's 3.4 M nodes takes 54 us from
 // the caller's tensors (84 before; its two copies are 7 us each).
 constexpr int kPackThreads = 256;
-template <typename D, typename Src>
-__global__ void __launch_bounds__(kPackThreads) pack_nodes(D* __restrict__ dst, const Src* __restrict__ src, Layout lay) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int cols = lay.C + 1, lane = threadIdx.x & 31;
-    const long long lines = (long long)(lay.S + 1) * (lay.R + 1);
-    const long long stride = (long long)gridDim.x * (kPackThreads / 32);
-    for (long long line = (long long)blockIdx.x * (kPackThreads / 32) + (threadIdx.x >> 5); line < lines; line += stride) {
-        const Src* const s = src + line * cols;
-        D* const d = dst + line * lay.Xp;
-#pragma unroll 4
-        for (int x = lane; x < lay.Xp; x += 32) d[x] = (x < cols) ? (D)s[x] : (D)0;
+constexpr int kPackSegment = 1024;
+struct PackShape {
+    int lanes;     // per segment: a power of two
+    int segments;  // per row
+    int length;    // nodes of a segment (the last one may be shorter)
+};
+inline PackShape pack_shape(const Layout& lay) {
+    PackShape p;
+    p.lanes = 4;
+    while (p.lanes < 32 && p.lanes < lay.Xp) p.lanes *= 2;
+    p.segments = (lay.Xp + kPackSegment - 1) / kPackSegment;
+    p.length = ((lay.Xp + p.segments - 1) / p.segments + 31) / 32 * 32;
+    return p;
+}
+// Calls row(line, x0, x1, lane) for every segment [x0, x1) of this thread's
+// groups.  The group width is a constant of the kernel: with a stride that is
+// not, the loads of a row are no longer issued together (c2's FP32 action 63 us
+// instead of 53).
+template <int LANES, class Row>
+__device__ __forceinline__ void pack_rows(const Layout& lay, const PackShape& p, Row row) {
+    constexpr int groups = kPackThreads / LANES;
+    const int lane = threadIdx.x & (LANES - 1);
+    const long long items = (long long)(lay.S + 1) * (lay.R + 1) * p.segments;
+    const long long stride = (long long)gridDim.x * groups;
+    for (long long i = (long long)blockIdx.x * groups + threadIdx.x / LANES; i < items; i += stride) {
+        const long long line = p.segments == 1 ? i : i / p.segments;
+        const int x0 = (int)(i - line * p.segments) * p.length;
+        row(line, x0, min(x0 + p.length, lay.Xp), lane);
     }
 }
 
-template <typename D, typename Src>
+template <int LANES, typename T>
 __global__ void __launch_bounds__(kPackThreads)
-    unpack_nodes(D* __restrict__ dst, const Src* __restrict__ src, Layout lay) {
+    pack_nodes(T* __restrict__ dst, const T* __restrict__ src, Layout lay, PackShape p) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int cols = lay.C + 1, lane = threadIdx.x & 31;
-    const long long lines = (long long)(lay.S + 1) * (lay.R + 1);
-    const long long stride = (long long)gridDim.x * (kPackThreads / 32);
-    for (long long line = (long long)blockIdx.x * (kPackThreads / 32) + (threadIdx.x >> 5); line < lines; line += stride) {
-        const Src* const s = src + line * lay.Xp;
-        D* const d = dst + line * cols;
+    const int cols = lay.C + 1;
+    pack_rows<LANES>(lay, p, [&](const long long line, const int x0, const int x1, const int lane) {
+        const T* const s = src + line * cols;
+        T* const d = dst + line * lay.Xp;
 #pragma unroll 4
-        for (int x = lane; x < cols; x += 32) d[x] = (D)s[x];
-    }
+        for (int x = x0 + lane; x < x1; x += LANES) d[x] = (x < cols) ? s[x] : T(0);
+    });
+}
+
+template <int LANES, typename T>
+__global__ void __launch_bounds__(kPackThreads)
+    unpack_nodes(T* __restrict__ dst, const T* __restrict__ src, Layout lay, PackShape p) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int cols = lay.C + 1;
+    pack_rows<LANES>(lay, p, [&](const long long line, const int x0, const int x1, const int lane) {
+        const T* const s = src + line * lay.Xp;
+        T* const d = dst + line * cols;
+        const int end = min(x1, cols);
+#pragma unroll 4
+        for (int x = x0 + lane; x < end; x += LANES) d[x] = s[x];
+    });
+}
+
+template <typename T>
+using PackKernel = void (*)(T*, const T*, Layout, PackShape);
+template <typename T>
+PackKernel<T> pack_kernel(const PackShape& p) {
+    return p.lanes == 32   ? pack_nodes<32, T>
+           : p.lanes == 16 ? pack_nodes<16, T>
+           : p.lanes == 8  ? pack_nodes<8, T>
+                           : pack_nodes<4, T>;
+}
+template <typename T>
+PackKernel<T> unpack_kernel(const PackShape& p) {
+    return p.lanes == 32   ? unpack_nodes<32, T>
+           : p.lanes == 16 ? unpack_nodes<16, T>
+           : p.lanes == 8  ? unpack_nodes<8, T>
+                           : unpack_nodes<4, T>;
 }
 
 // Element conductivities: flat FP64 (S, R, C) -> padded FP64 and FP32 (S, R, Xe).
