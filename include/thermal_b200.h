@@ -127,7 +127,8 @@ int tb_system_info(const tb_system* system, int64_t* nodes, int64_t* device_byte
 
 /* y = A x, A = where(free, K (x * free) + R x, x): the FP32 low action
  * (reference apply_low, operator.py:349-361; hex_q1.cpp:503-509) and the FP64
- * high action (apply_high, operator.py:308-316; thermal_hex.hpp:32-39). */
+ * high action (apply_high, operator.py:308-316; thermal_hex.hpp:32-39).  When
+ * an action fails, y is left as it was. */
 int tb_apply_f32(tb_system* system, const float* x, float* y);
 int tb_apply_f64(tb_system* system, const double* x, double* y);
 int tb_apply_f32_device(tb_system* system, const float* d_x, float* d_y);

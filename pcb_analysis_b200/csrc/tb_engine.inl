@@ -843,7 +843,7 @@ int engine_collect(tb_engine* e, long long ticket, double* x, tb_mpir_result* re
         void* tmp = nullptr;
         TB_CUDA(cudaMallocFromPoolAsync(&tmp, sizeof(double) * (size_t)L.N, e->pool, e->io));
         unpack_kernel<double>(pack_shape(L))<<<pack_grid(L, e->sms), kPackThreads, 0, e->io>>>(
-            static_cast<double*>(tmp), b->inst.x64, L, pack_shape(L));
+            static_cast<double*>(tmp), b->inst.x64, L, pack_shape(L), nullptr);
         TB_CUDA(cudaGetLastError());
         e->kernel_launches += 1;
         TB_CUDA(cudaMemcpyAsync(x, tmp, sizeof(double) * (size_t)L.N, cudaMemcpyDeviceToHost, e->io));

@@ -1362,24 +1362,26 @@ int load_nodes(tb_system* s, T* dst, const T* src, bool src_on_device) {
     return TB_OK;
 }
 
-// `pdl`: launched as a programmatic dependent of the kernel that wrote `src`.
+// `pdl`: launched as a programmatic dependent of the kernel that wrote `src`;
+// `err`: a device error word that, when set, leaves a device `dst` untouched.
 template <typename T>
-int store_nodes(tb_system* s, T* dst, const T* src, bool dst_on_device, bool pdl = false) {
+int store_nodes(tb_system* s, T* dst, const T* src, bool dst_on_device, bool pdl = false, const int* err = nullptr) {
     const Layout& L = s->lay;
     const int nb = pack_grid(L, s->sms);
     if (dst_on_device) {
         if (pdl) {
             TB_CUDA(launch_pdl(unpack_kernel<T>(pack_shape(L)), dim3(nb), dim3(kPackThreads), 0, s->stream, dst, src, L,
-                               pack_shape(L)));
+                               pack_shape(L), err));
         } else {
-            unpack_kernel<T>(pack_shape(L))<<<nb, kPackThreads, 0, s->stream>>>(dst, src, L, pack_shape(L));
+            unpack_kernel<T>(pack_shape(L))<<<nb, kPackThreads, 0, s->stream>>>(dst, src, L, pack_shape(L), err);
             TB_CUDA(cudaGetLastError());
         }
         s->kernel_launches += 1;
         return TB_OK;
     }
     TB_CHECK(ensure_stage(s, sizeof(T) * (size_t)L.N));
-    unpack_kernel<T>(pack_shape(L))<<<nb, kPackThreads, 0, s->stream>>>(static_cast<T*>(s->stage), src, L, pack_shape(L));
+    unpack_kernel<T>(pack_shape(L))<<<nb, kPackThreads, 0, s->stream>>>(static_cast<T*>(s->stage), src, L, pack_shape(L),
+                                                                     nullptr);
     TB_CUDA(cudaGetLastError());
     s->kernel_launches += 1;
     TB_CHECK(device_to_host(s, dst, s->stage, sizeof(T) * L.N));
@@ -2486,7 +2488,7 @@ static int apply_any(tb_system* s, const void* x, void* y, bool f64, bool dev, b
         const ApplyParams<float> P = apply_params<float>(s, s->p32, s->q32, nullptr);
         TB_CHECK((launch_apply<float, MODE_OPERATOR, EPI_STORE>(s, P, true)));
         if (dev) {  // one wait for the three kernels and the staging's error word
-            TB_CHECK(store_nodes<float>(s, static_cast<float*>(y), s->q32, true, true));
+            TB_CHECK(store_nodes<float>(s, static_cast<float*>(y), s->q32, true, true, s->stage_err));
             s->kernel_launches += 1;
             return check_stage(s);
         }

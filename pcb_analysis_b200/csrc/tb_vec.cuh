@@ -82,11 +82,14 @@ __global__ void __launch_bounds__(kPackThreads)
     });
 }
 
+// `err` (null: none): the error word of the kernel that wrote `src`; when it is
+// set, src is incomplete and dst is left as it is.
 template <int LANES, typename T>
 __global__ void __launch_bounds__(kPackThreads)
-    unpack_nodes(T* __restrict__ dst, const T* __restrict__ src, Layout lay, PackShape p) {
+    unpack_nodes(T* __restrict__ dst, const T* __restrict__ src, Layout lay, PackShape p, const int* err) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (err != nullptr && *err != 0) return;
     const int cols = lay.C + 1;
     pack_rows<LANES>(lay, p, [&](const long long line, const int x0, const int x1, const int lane) {
         const T* const s = src + line * lay.Xp;
@@ -107,7 +110,9 @@ PackKernel<T> pack_kernel(const PackShape& p) {
                            : pack_nodes<4, T>;
 }
 template <typename T>
-PackKernel<T> unpack_kernel(const PackShape& p) {
+using UnpackKernel = void (*)(T*, const T*, Layout, PackShape, const int*);
+template <typename T>
+UnpackKernel<T> unpack_kernel(const PackShape& p) {
     return p.lanes == 32   ? unpack_nodes<32, T>
            : p.lanes == 16 ? unpack_nodes<16, T>
            : p.lanes == 8  ? unpack_nodes<8, T>

@@ -55,3 +55,21 @@ def test_a_stage_wait_that_runs_out_is_reported_and_the_system_stays_usable(plan
         again = dev.solve_mpir(rhs, CONFIG)
         np.testing.assert_array_equal(again["solution"], solved["solution"])
         assert again["history"] == solved["history"]
+
+
+@pytest.mark.parametrize("plan", [(0, 16, 1, 0, 0), (2, 8, 1, 0, 0)])
+def test_an_action_that_fails_leaves_the_callers_tensor_alone(plan) -> None:
+    import torch
+
+    arrays, _ = _arrays()
+    with DeviceSystem(**arrays) as dev:
+        dev.apply_plan = plan
+        x = torch.randn(dev.size, generator=torch.Generator().manual_seed(2)).cuda()
+        y = torch.full_like(x, 7.0)
+        dev.set_stage_test(64)
+        with pytest.raises(TimeoutError, match="staged tiles"):
+            dev.apply_f32_device(x, y)
+        assert bool((y == 7.0).all())
+        dev.set_stage_test(0)
+        dev.apply_f32_device(x, y)
+        np.testing.assert_array_equal(y.cpu().numpy(), dev.apply_f32(x.cpu().numpy()))
