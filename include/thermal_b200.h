@@ -180,8 +180,28 @@ int tb_solve_pcg_f64_ml_device(tb_system* system, const double* d_rhs, double* d
  * timeout and returns with nothing in flight, and the apply or solve fails
  * with TB_ETIMEOUT.  0 restores normal staging.  Affects launch plans with
  * tensor-copy staging (tb_set_apply_plan), and the cooperative PCG kernel of
- * small boards, whose first block then posts nothing. */
+ * small boards, one of whose blocks then posts nothing (TB_TEST_PCG_MUTE). */
 int tb_set_stage_test(tb_system* system, int32_t polls);
+
+/* Test only: switches that reach launch forms and failure paths on small
+ * boards.
+ *   TB_TEST_PCG_MUTE: while tb_set_stage_test is on, the words that one block
+ *     of the cooperative PCG kernel does not post: 1 direction, 2 p.q, 4 patch
+ *     sums, 8 coarse solution, 16 r.z, or a sum of them; 0 (default): all.
+ *   TB_TEST_PCG_MUTE_BLOCK: which block (default 0).
+ *   TB_TEST_PCG_REFUSE: 1: the kernel's buffers are asked for in a size that no
+ *     device has; 2: its launch in a grid that does not fit; 0: neither.
+ *   TB_TEST_PCG_SLICE: iterations of one launch of the kernel; 0: the default.
+ *   TB_TEST_WIDE_COLUMNS: node columns from which every multilevel level runs
+ *     with one thread per column; -1: the default thresholds. */
+enum {
+    TB_TEST_PCG_MUTE = 0,
+    TB_TEST_PCG_MUTE_BLOCK = 1,
+    TB_TEST_PCG_REFUSE = 2,
+    TB_TEST_PCG_SLICE = 3,
+    TB_TEST_WIDE_COLUMNS = 4
+};
+int tb_set_test(tb_system* system, int32_t what, int64_t value);
 
 /* Launch form of the multilevel preconditioner's fine pass in the inner FP32
  * PCG iterations (no reference counterpart; the reference's preconditioners

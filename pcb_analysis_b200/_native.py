@@ -234,6 +234,7 @@ _SIGNATURES: dict[str, tuple[Any, list[Any]]] = {
     ),
     "tb_set_timing": (ctypes.c_int, [_VP, _I32]),
     "tb_set_stage_test": (ctypes.c_int, [_VP, _I32]),
+    "tb_set_test": (ctypes.c_int, [_VP, _I32, ctypes.c_int64]),
     "tb_set_ml_staging": (ctypes.c_int, [_VP, _I32]),
     "tb_get_ml_staging": (ctypes.c_int, [_VP, ctypes.POINTER(ctypes.c_int32)]),
     "tb_get_timing": (ctypes.c_int, [_VP, _c_double_p, ctypes.POINTER(ctypes.c_int64)]),
@@ -578,6 +579,12 @@ class DeviceSystem:
         """Test only: make the tensor-copy stage waits run out (tb_set_stage_test)."""
 
         check(self._lib.tb_set_stage_test(self.handle, int(polls)))
+
+    def set_test(self, what: str, value: int) -> None:
+        """Test only: the switches of tb_set_test by name."""
+
+        names = ("pcg_mute", "pcg_mute_block", "pcg_refuse", "pcg_slice", "wide_columns")
+        check(self._lib.tb_set_test(self.handle, names.index(what), int(value)))
 
     @property
     def ml_staging(self) -> bool:

@@ -119,9 +119,10 @@ cudaError_t ml_launch(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block,
 // and on 2048 cells ml_down of level 1 118 / 108 us, ml_up 160 / 85 us, the
 // fine pass 397 us with the pre-smoothing in its blocks against 344 + 14 us.
 constexpr long long kMlWideDown = 130000, kMlWideUp = 40000, kMlWidePre = 25000;
-bool ml_wide_down(const MLGrid& g) { return g.plane >= kMlWideDown; }
-bool ml_wide_up(const MLGrid& g) { return g.plane >= kMlWideUp; }
-bool ml_wide_pre(const tb_system* s) { return s->ml.size() > 1 && s->ml[0].g.plane >= kMlWidePre; }
+long long ml_wide_from(const tb_system* s, long long columns) { return s->test_wide >= 0 ? s->test_wide : columns; }
+bool ml_wide_down(const tb_system* s, const MLGrid& g) { return g.plane >= ml_wide_from(s, kMlWideDown); }
+bool ml_wide_up(const tb_system* s, const MLGrid& g) { return g.plane >= ml_wide_from(s, kMlWideUp); }
+bool ml_wide_pre(const tb_system* s) { return s->ml.size() > 1 && s->ml[0].g.plane >= ml_wide_from(s, kMlWidePre); }
 dim3 ml_column_grid(const MLGrid& g) { return dim3((unsigned)((g.plane + kMlWideThreads - 1) / kMlWideThreads)); }
 
 int ml_vcycle_kernels(const tb_system* s) { return 2 * (int)s->ml.size() - 1 + (ml_wide_pre(s) ? 1 : 0); }
@@ -147,7 +148,7 @@ cudaError_t ml_launch_down(tb_system* s, int l, bool pdl, const SolveCtl* ctl) {
     const tb_system::MLLevel& dn = s->ml[l + 1];
     const bool dense = l + 2 == (int)s->ml.size();
     const dim3 grid = ml_level_grid(lv.g);
-    if (ml_wide_down(lv.g)) {
+    if (ml_wide_down(s, lv.g)) {
         constexpr int NP = ROUNDS == 1 ? 9 : (ROUNDS == 2 ? 18 : 33);
         return ml_launch(pdl, ml_down_wide<NP, B>, dim3(ml_cdiv(lv.g.nx, kMlWideX), ml_cdiv(lv.g.ny, kMlWideY)),
                          dim3(kMlWideThreads), s->stream, (const float*)lv.st, (const float*)lv.R, (const float*)lv.x,
@@ -175,7 +176,7 @@ cudaError_t ml_launch_up(tb_system* s, int l, int mode, bool pdl) {
     const tb_system::MLLevel& lv = s->ml[l];
     const tb_system::MLLevel& dn = s->ml[l + 1];
     SolveCtl* const state = mode == ML_ONLY ? nullptr : s->ctl;
-    if (ml_wide_up(lv.g)) {
+    if (ml_wide_up(s, lv.g)) {
         constexpr int NP = ROUNDS == 1 ? 9 : (ROUNDS == 2 ? 18 : 33);
         return ml_launch(pdl, l == 0 ? ml_up_wide<NP, B, true> : ml_up_wide<NP, B, false>,
                          ml_column_grid(lv.g), dim3(kMlWideThreads), s->stream, (const float*)lv.az,

@@ -69,6 +69,9 @@ constexpr int kResTouched = 1024;  // patches a block touches at most
 constexpr int kResSlots = 16;      // blocks that touch one patch row at most
 constexpr int kResPolls = 1 << 22; // polls of a post before a block gives up (seconds)
 
+// The kinds of words the blocks post (ResidentParams::mute).
+enum { kResDirection = 1, kResPq = 2, kResPatchSums = 4, kResCoarse = 8, kResRz = 16 };
+
 struct ResidentParams {
     float *p, *x, *r;
     const float* dinv;
@@ -84,7 +87,9 @@ struct ResidentParams {
     int chunk;  // nodes of a block
     int limit;  // iterations of one launch
     int polls;
-    int mute;   // test only: block 0 posts nothing, so every wait runs out
+    // test only: words (kResDirection ..) that block `mute_block` does not post,
+    // so that the waits for them run out
+    int mute, mute_block;
     // two-level (null minv: Jacobi)
     CoarseLayout cl;
     const float* minv;
@@ -220,6 +225,13 @@ __device__ __forceinline__ double res_warp_sum(double v) {
     return v;
 }
 
+// MUTE: the instantiations of the test switch (a test in the loop of the others
+// costs a tenth of a small board's iteration).
+template <bool MUTE>
+__device__ __forceinline__ bool res_muted(const ResidentParams& P, const int kind) {
+    return MUTE && (P.mute & kind) != 0 && (int)blockIdx.x == P.mute_block;
+}
+
 // One exchange of NA sums.  Warp k merges the block's warps for sum k, posts
 // it (FP64, as two FP32 words: the sum rounded and what is left) and gathers
 // every block's, five posts a lane; warp 0 then runs fin(totals) on all its
@@ -231,9 +243,9 @@ struct ResShared {
     double red[3][kResThreads / 32], tot[3];
     int ok[3], go;
 };
-template <int NA, class Fin>
-__device__ __forceinline__ bool res_exchange(const ResidentParams& P, unsigned long long* posts, unsigned int tag,
-                                             const Acc32 (&acc)[NA], ResShared& sh, Fin&& fin) {
+template <int NA, bool MUTE, class Fin>
+__device__ __forceinline__ bool res_exchange(const ResidentParams& P, unsigned long long* posts, int kind,
+                                             unsigned int tag, const Acc32 (&acc)[NA], ResShared& sh, Fin&& fin) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, blocks = gridDim.x;
 #pragma unroll
     for (int k = 0; k < NA; ++k) {
@@ -245,7 +257,7 @@ __device__ __forceinline__ bool res_exchange(const ResidentParams& P, unsigned l
         const double mine = res_warp_sum(lane < kResThreads / 32 ? sh.red[warp][lane] : 0.0);
         // copy c of this sum's posts: [block] pairs
         auto column = [&](const int c) { return posts + ((size_t)c * blocks * NA + warp) * 2; };
-        if (lane < kResCopies && !(P.mute && blockIdx.x == 0)) {
+        if (lane < kResCopies && !res_muted<MUTE>(P, kind)) {
             const float hi = (float)mine;
             res_post2(column(lane) + (size_t)blockIdx.x * 2 * NA, tag, hi, (float)(mine - (double)hi));
         }
@@ -298,7 +310,7 @@ inline size_t resident_smem(int trows, int tcols, int chunk, int Xp) {
     return sizeof(float) * (tl + 3 * (size_t)resident_segment(chunk, Xp));
 }
 
-template <int NODES, bool TL>
+template <int NODES, bool TL, bool MUTE>
 __global__ void __launch_bounds__(kResThreads, 1) resident_pcg(const __grid_constant__ ResidentParams P) {
     constexpr int NA = TL ? 3 : 2;
     __shared__ ResShared sh;
@@ -389,7 +401,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_pcg(const __grid_cons
             const int at = t + k * kResThreads;
             if (own[k]) {
                 const float u = d[k] > 0.f ? p[k] : 0.f;  // the free part
-                res_post(P.halo + base + at, tag, u);
+                if (!res_muted<MUTE>(P, kResDirection)) res_post(P.halo + base + at, tag, u);
                 s_h[seg + Xp + 1 + at] = u;
             }
         }
@@ -437,7 +449,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_pcg(const __grid_cons
             q[k] = (s0 + s1) + s2;
             apq[0].add_product(p[k], q[k]);
         }
-        ok = res_exchange<1>(P, P.posts, tag, apq, sh, [&](const double (&tot)[1]) {
+        ok = res_exchange<1, MUTE>(P, P.posts, kResPq, tag, apq, sh, [&](const double (&tot)[1]) {
             const double alpha = s_ctl.rz / tot[0];
             if (t != 0) return;
             s_ctl.pq = tot[0];
@@ -478,7 +490,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_pcg(const __grid_cons
                 double v = (double)s;
 #pragma unroll
                 for (int off = 8; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off, 16);
-                if (real && lane == 0)
+                if (real && lane == 0 && !res_muted<MUTE>(P, kResPatchSums))
                     res_post(P.part + (size_t)(blk - first / P.chunk) * P.cl.ld + (size_t)pr * P.cl.nbx + pc, tag, (float)v);
             }
             // R of the tile's columns and rows
@@ -520,12 +532,12 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_pcg(const __grid_cons
                 u += __shfl_xor_sync(0xffffffffu, u, 1);
                 const int row = 4 * rq + (h8 ? 2 : 0) + (h4 ? 1 : 0);
                 if (real && (cg & 3) == 0 && row < nrow) {
-                    res_post(P.c + (size_t)tile_x * P.cl.ld + row0 + row, tag, u);
+                    if (!res_muted<MUTE>(P, kResCoarse)) res_post(P.c + (size_t)tile_x * P.cl.ld + row0 + row, tag, u);
                     au[NA - 1].add_product(s_R[P.tcols + row], u);
                 }
             }
         }
-        ok = res_exchange<NA>(P, P.posts + 2 * kResCopies * gridDim.x, tag, au, sh, [&](const double (&tot)[NA]) {
+        ok = res_exchange<NA, MUTE>(P, P.posts + 2 * kResCopies * gridDim.x, kResRz, tag, au, sh, [&](const double (&tot)[NA]) {
             if (t != 0) return;
             const double rzn = TL ? tot[1] + tot[NA - 1] : tot[1], ratio = rzn / s_ctl.rz;
             s_ctl.iterations += 1;

@@ -5,9 +5,10 @@ constexpr int kResLimit = 512;      // iterations of one launch (a few milliseco
 constexpr int kResMinChunk = 128;   // nodes of a block at least
 
 using ResidentKernel = void (*)(const ResidentParams);
+template <bool MUTE>
 ResidentKernel resident_kernel(int nodes, bool tl) {
-    if (nodes == 1) return tl ? resident_pcg<1, true> : resident_pcg<1, false>;
-    return tl ? resident_pcg<2, true> : resident_pcg<2, false>;
+    if (nodes == 1) return tl ? resident_pcg<1, true, MUTE> : resident_pcg<1, false, MUTE>;
+    return tl ? resident_pcg<2, true, MUTE> : resident_pcg<2, false, MUTE>;
 }
 
 void free_resident(tb_system* s) {
@@ -44,15 +45,16 @@ int resident_setup(tb_system* s) {
     const size_t smem = resident_smem(trows, tcols, chunk, L.Xp);
     int optin = 0;
     TB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
-    const ResidentKernel kernel = resident_kernel(nodes, tl);
-    cudaFuncAttributes fa{};
-    TB_CUDA(cudaFuncGetAttributes(&fa, kernel));
-    if (fa.sharedSizeBytes + smem > (size_t)optin) return TB_OK;
-    TB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 optin - (int)fa.sharedSizeBytes));
-    int per_sm = 0;
-    TB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kResThreads, smem));
-    if (per_sm < 1) return TB_OK;
+    for (const ResidentKernel kernel : {resident_kernel<false>(nodes, tl), resident_kernel<true>(nodes, tl)}) {
+        cudaFuncAttributes fa{};
+        TB_CUDA(cudaFuncGetAttributes(&fa, kernel));
+        if (fa.sharedSizeBytes + smem > (size_t)optin) return TB_OK;
+        TB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     optin - (int)fa.sharedSizeBytes));
+        int per_sm = 0;
+        TB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kResThreads, smem));
+        if (per_sm < 1) return TB_OK;
+    }
     int slots = 0;
     if (tl) {
         // blocks that touch one patch row: from the one that holds its first node on
@@ -73,7 +75,7 @@ int resident_setup(tb_system* s) {
     // tagged words: the direction, the sums, the patch sums, the coarse solution; and the next tag
     const long long sums = 8LL * kResCopies * blocks, parts = tl ? (long long)slots * s->cl.ld : 0, cs = (long long)tiles_x * s->cl.ld;
     s->res_word_count = L.L + sums + parts + cs + 1;  // L is a multiple of 4: the sums' pairs stay 16-byte aligned
-    TB_CHECK(alloc_n(s, &s->res_words, s->res_word_count));
+    TB_CHECK(alloc_n(s, &s->res_words, s->test_refuse == 1 ? 1LL << 50 : s->res_word_count));
     resident_rows<<<grid_for(L.L, 128, s->sms * 16), 128, 0, s->stream>>>(
         s->res_rows, s->kin64, s->kz64, s->rf64, s->dims64, s->dims64 + L.S, s->dims64 + L.S + L.C, L);
     TB_CUDA(cudaGetLastError());
@@ -95,7 +97,7 @@ int resident_setup(tb_system* s) {
     P.tag = reinterpret_cast<unsigned int*>(P.c + cs);
     P.err = s->stage_err;
     P.chunk = chunk;
-    P.limit = kResLimit;
+    P.limit = s->test_slice > 0 ? s->test_slice : kResLimit;
     P.polls = kResPolls;
     P.cl = s->cl;
     P.minv = tl ? s->coarse_inv32 : nullptr;
@@ -127,12 +129,14 @@ int run_resident(tb_system* s, SolveCtl* out) {
     ResidentParams P = s->res_params;
     if (s->maps[0].test_polls > 0) {
         P.polls = s->maps[0].test_polls;
-        P.mute = 1;
+        P.mute = s->test_mute != 0 ? s->test_mute : ~0;
+        P.mute_block = s->test_mute_block;
     }
-    const ResidentKernel kernel = resident_kernel(s->res_nodes, P.minv != nullptr);
+    const bool tl = P.minv != nullptr;
+    const ResidentKernel kernel = P.mute ? resident_kernel<true>(s->res_nodes, tl) : resident_kernel<false>(s->res_nodes, tl);
     void* args[] = {&P};
     for (long long n = 0;; ++n) {
-        TB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(s->res_blocks),
+        TB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(s->test_refuse == 2 ? 1 << 16 : s->res_blocks),
                                             dim3(kResThreads), args, s->res_smem, s->stream));
         s->kernel_launches += 1;
         TB_CHECK(read_ctl(s, out));

@@ -188,6 +188,9 @@ struct tb_system {
     unsigned long long* res_words = nullptr;
     long long res_word_count = 0;
     ResidentParams res_params{};
+    // test switches (tb_set_test)
+    int test_mute = 0, test_mute_block = 0, test_refuse = 0, test_slice = 0;
+    long long test_wide = -1;
     // problem terms of a system made by tb_system_create_problem (flat node
     // order): node flags, loads, Robin terms, C / dt, fixed values, and each
     // convection boundary's lumped weights for its removed heat
@@ -2700,6 +2703,27 @@ int tb_set_stage_test(tb_system* s, int32_t polls) {
     for (ApplyMaps& m : s->maps) m.test_polls = polls;
     s->ml_maps.test_polls = polls;
     for (int k = 0; k < 2; ++k) {  // the graphs hold the maps by value
+        release_slot(s->slots32[k]);
+        release_slot(s->slots64[k]);
+    }
+    return TB_OK;
+}
+
+int tb_set_test(tb_system* s, int32_t what, int64_t value) {
+    if (!s) return fail(TB_EINVAL, "system is NULL");
+    if (value < (what == TB_TEST_WIDE_COLUMNS ? -1 : 0) || value > INT32_MAX) return fail(TB_EINVAL, "value is out of range");
+    TB_CUDA(cudaSetDevice(s->device));
+    TB_CUDA(cudaStreamSynchronize(s->stream));
+    switch (what) {
+        case TB_TEST_PCG_MUTE: s->test_mute = (int)value; break;
+        case TB_TEST_PCG_MUTE_BLOCK: s->test_mute_block = (int)value; break;
+        case TB_TEST_PCG_REFUSE: s->test_refuse = (int)value; break;
+        case TB_TEST_PCG_SLICE: s->test_slice = (int)value; break;
+        case TB_TEST_WIDE_COLUMNS: s->test_wide = value; break;
+        default: return fail(TB_EINVAL, "unknown test switch %d", (int)what);
+    }
+    free_resident(s);  // made again with the new switches
+    for (int k = 0; k < 2; ++k) {  // the graphs hold the launch forms
         release_slot(s->slots32[k]);
         release_slot(s->slots64[k]);
     }

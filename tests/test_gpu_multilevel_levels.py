@@ -7,7 +7,10 @@ level 1's pre-smoothing runs in the fine pass's blocks or as a kernel.  Each
 form is held to a NumPy FP64 restatement of M^-1 r = T^-1 r + Z_1 V_1(Z_1^T r)
 built on the device's own coarse stencils (which other tests pin to the
 Galerkin products), so that boards too wide for an assembled operator can be
-checked.  Tolerance: 1e-4 of the result's norm, what the assembled restatement
+checked.  The boards of test_level_forms reach their forms by size; a test
+switch has every level of the boards of test_wide_forms run in its wide form,
+so that each plane count's kernel is reached by a board of modest size.
+Tolerance: 1e-4 of the result's norm, what the assembled restatement
 is held to.
 """
 
@@ -106,10 +109,34 @@ def _vcycle(levels, inverse, grids, r, l=0):
     ],
 )
 def test_level_forms(ns_local, slabs, rows, cols, fixed):
-    problem = _board(ns_local, slabs, rows, cols, fixed)
-    op = ns_local.MatrixFreeThermalOperator(problem, preconditioner="multilevel")
+    _check(ns_local, slabs, rows, cols, fixed)
+
+
+# Level 1 is more than 200 columns long, so that the aggregates below it are 2 x 2
+# (the wide forms are built for those) but for the last board's 4 x 4.
+@pytest.mark.parametrize(
+    "slabs, rows, cols, fixed",
+    [
+        (8, 811, 21, False),    # nine planes, the most of the nine-plane kernels
+        (9, 23, 817, True),     # ten: the next kernels up
+        (16, 811, 30, True),    # seventeen: the most of the seventeen-plane pre-smoothing
+        (17, 26, 809, False),   # eighteen: the most of the eighteen-plane kernels
+        (18, 812, 17, True),    # nineteen
+        (32, 811, 22, False),   # thirty-three
+        (19, 66, 90, True),     # 4 x 4 aggregates: only the pre-smoothing is wide
+    ],
+)
+def test_wide_forms(ns_local, slabs, rows, cols, fixed):
+    _check(ns_local, slabs, rows, cols, fixed, wide=True)
+
+
+def _check(ns, slabs, rows, cols, fixed, wide=False):
+    problem = _board(ns, slabs, rows, cols, fixed)
+    op = ns.MatrixFreeThermalOperator(problem, preconditioner="multilevel")
     try:
         system = op.device_system
+        if wide:
+            system.set_test("wide_columns", 0)
         grids = system.multilevel_grids()
         levels = [system.multilevel_stencil(l + 1).astype(np.float64) for l in range(len(grids) - 1)]
         inverse = system.coarse()[1]

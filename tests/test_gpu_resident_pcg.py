@@ -136,3 +136,30 @@ def test_a_wait_that_runs_out_is_reported(ns_local):
     finally:
         op.close()
     np.testing.assert_array_equal(before["solution"], after["solution"])
+
+
+@pytest.mark.parametrize(
+    "preconditioner, words",
+    [("jacobi", 1), ("jacobi", 2), ("jacobi", 16), ("two-level", 1), ("two-level", 2), ("two-level", 4),
+     ("two-level", 8), ("two-level", 16), ("two-level", 0)],
+)
+@pytest.mark.parametrize("block", [0, 7])
+def test_every_wait_that_runs_out_is_reported(ns_local, preconditioner, words, block):
+    """One block keeps back one kind of word: direction, p.q, patch sums, coarse
+    solution or r.z (0: all of them)."""
+
+    op = ns_local.MatrixFreeThermalOperator(workloads.board_c1(0, None, 40, 48), preconditioner=preconditioner)
+    try:
+        system = op.device_system
+        rhs = op.build_rhs(op.default_reference_temperature())
+        before = system.solve_mpir(rhs, CONFIG)
+        system.set_test("pcg_mute", words)
+        system.set_test("pcg_mute_block", block)
+        system.set_stage_test(64)
+        with pytest.raises(TimeoutError):
+            system.solve_mpir(rhs, CONFIG)
+        system.set_stage_test(0)
+        after = system.solve_mpir(rhs, CONFIG)
+    finally:
+        op.close()
+    np.testing.assert_array_equal(before["solution"], after["solution"])
