@@ -71,11 +71,17 @@ int resident_setup(tb_system* s) {
         const int touched = std::min(prows, lines / s->cl.b + lines / (L.R + 1) + 3) * s->cl.nbx;
         if (slots > kResSlots || touched > kResTouched) return TB_OK;
     }
-    TB_CHECK(alloc_n(s, &s->res_rows, kResRow * L.L));
+    // Without the memory for them the solve runs on the graph-captured kernels.
+    const auto refused = [s]() {
+        free_resident(s);
+        s->res_state = -1;
+        return TB_OK;
+    };
+    if (alloc_n(s, &s->res_rows, kResRow * L.L) != TB_OK) return refused();
     // tagged words: the direction, the sums, the patch sums, the coarse solution; and the next tag
     const long long sums = 8LL * kResCopies * blocks, parts = tl ? (long long)slots * s->cl.ld : 0, cs = (long long)tiles_x * s->cl.ld;
     s->res_word_count = L.L + sums + parts + cs + 1;  // L is a multiple of 4: the sums' pairs stay 16-byte aligned
-    TB_CHECK(alloc_n(s, &s->res_words, s->test_refuse == 1 ? 1LL << 50 : s->res_word_count));
+    if (alloc_n(s, &s->res_words, s->test_refuse == 1 ? 1LL << 50 : s->res_word_count) != TB_OK) return refused();
     resident_rows<<<grid_for(L.L, 128, s->sms * 16), 128, 0, s->stream>>>(
         s->res_rows, s->kin64, s->kz64, s->rf64, s->dims64, s->dims64 + L.S, s->dims64 + L.S + L.C, L);
     TB_CUDA(cudaGetLastError());
@@ -118,6 +124,10 @@ int resident_setup(tb_system* s) {
 bool resident_wanted(const tb_system* s) { return !s->timing && !s->plan_set && s->physics == 0 && s->precond <= 1; }
 
 // The inner PCG from a prepared start (as run_pcg) on the cooperative kernel.
+// A launch that the runtime refuses (the device's SMs shared out to several
+// clients, say) leaves the vectors and the scalars as the last one left them,
+// with `state` running: the caller goes on from there with the graph-captured
+// kernels.
 int run_resident(tb_system* s, SolveCtl* out) {
     if (s->res_fresh) {  // nothing exchanged yet, or a run that was given up: words without tags, the first tag 1
         TB_CUDA(cudaMemsetAsync(s->res_words, 0, sizeof(unsigned long long) * (size_t)s->res_word_count, s->stream));
@@ -136,8 +146,15 @@ int run_resident(tb_system* s, SolveCtl* out) {
     const ResidentKernel kernel = P.mute ? resident_kernel<true>(s->res_nodes, tl) : resident_kernel<false>(s->res_nodes, tl);
     void* args[] = {&P};
     for (long long n = 0;; ++n) {
-        TB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(s->test_refuse == 2 ? 1 << 16 : s->res_blocks),
-                                            dim3(kResThreads), args, s->res_smem, s->stream));
+        if (cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel),
+                                        dim3(s->test_refuse == 2 ? 1 << 16 : s->res_blocks), dim3(kResThreads), args,
+                                        s->res_smem, s->stream) != cudaSuccess) {
+            cudaGetLastError();  // an error that outlives the launch meets the next call
+            free_resident(s);
+            s->res_state = -1;
+            TB_CHECK(read_ctl(s, out));
+            return TB_OK;
+        }
         s->kernel_launches += 1;
         TB_CHECK(read_ctl(s, out));
         if (out->state != ST_RUNNING) break;

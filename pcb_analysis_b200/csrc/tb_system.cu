@@ -877,7 +877,10 @@ int kernels_per_iteration(const tb_system* s, bool f64) {
 int run_pcg(tb_system* s, bool f64, SolveCtl* out) {
     if (!f64 && resident_wanted(s)) {
         TB_CHECK(resident_setup(s));
-        if (s->res_state == 1) return run_resident(s, out);
+        if (s->res_state == 1) {
+            TB_CHECK(run_resident(s, out));
+            if (out->state != ST_RUNNING) return TB_OK;
+        }
     }
     TB_CHECK(ensure_slots(s, f64));
     ChunkSlot* slots = f64 ? s->slots64 : s->slots32;

@@ -163,3 +163,33 @@ def test_every_wait_that_runs_out_is_reported(ns_local, preconditioner, words, b
     finally:
         op.close()
     np.testing.assert_array_equal(before["solution"], after["solution"])
+
+
+@pytest.mark.parametrize("preconditioner", ["jacobi", "two-level"])
+@pytest.mark.parametrize("refused", [1, 2])
+def test_a_refused_kernel_leaves_the_solve_to_the_graph_kernels(ns_local, preconditioner, refused):
+    """Its buffers (1) or its cooperative launch (2) are refused by the runtime."""
+
+    problem = workloads.board_c1(0, None, 40, 48)
+    out = []
+    for graph in (False, True):
+        op = ns_local.MatrixFreeThermalOperator(problem, preconditioner=preconditioner)
+        try:
+            system = op.device_system
+            rhs = op.build_rhs(op.default_reference_temperature())
+            if graph:
+                system.apply_plan = system.apply_plan
+            else:
+                system.set_test("pcg_refuse", refused)
+            out.append(system.solve_mpir(rhs, CONFIG))
+            if not graph:  # allowed again: the kernel is taken up again
+                system.set_test("pcg_refuse", 0)
+                launches = system.launch_count()
+                again = system.solve_mpir(rhs, CONFIG)
+                assert again["converged"]
+                assert system.launch_count() - launches < 1000
+        finally:
+            op.close()
+    assert out[0]["converged"]
+    np.testing.assert_array_equal(out[0]["solution"], out[1]["solution"])
+    assert out[0]["history"] == out[1]["history"]
