@@ -45,9 +45,9 @@
 // tile per block, not a row of tiles: a block then reads some 500 words of R
 // instead of 6,000, which took 7 us an iteration.)
 //
-// Every wait is bounded: a block whose wait runs out sets the error word and
-// the solve state and leaves; the others, which then miss its next words, do
-// the same.
+// Every wait is bounded: a block whose wait runs out sets the error word, which
+// the host reads after every launch, and leaves; the others, which then miss its
+// next words, do the same.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -599,7 +599,6 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_pcg(const __grid_cons
     if (t != 0) return;
     if (!ok) {
         atomicExch(P.err, 1);
-        P.ctl->state = ST_STAGE_TIMEOUT;
     } else if (blk == 0) {
         P.clock->total_ns += s_op_ns;
         P.clock->count += (unsigned long long)(s_ctl.applications - P.ctl->applications);

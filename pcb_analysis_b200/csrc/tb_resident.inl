@@ -156,14 +156,16 @@ int run_resident(tb_system* s, SolveCtl* out) {
             return TB_OK;
         }
         s->kernel_launches += 1;
+        TB_CUDA(cudaMemcpyAsync(s->h_err, s->stage_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
         TB_CHECK(read_ctl(s, out));
-        if (out->state != ST_RUNNING) break;
+        // The error word decides, whatever the state says: block 0, which writes
+        // the scalars, may have had all it waited for when another block gave up.
+        if (*s->h_err != 0) {
+            s->res_fresh = true;
+            TB_CUDA(cudaMemsetAsync(s->stage_err, 0, sizeof(int), s->stream));
+            return fail(TB_ETIMEOUT, "a block of the PCG kernel gave up waiting for the others");
+        }
+        if (out->state != ST_RUNNING) return TB_OK;
         if (n > (1LL << 40)) return fail(TB_ETIMEOUT, "PCG did not stop");
     }
-    if (out->state == ST_STAGE_TIMEOUT) {
-        s->res_fresh = true;
-        return check_stage(s) == TB_OK ? fail(TB_ETIMEOUT, "a block of the PCG kernel gave up waiting for the others")
-                                       : TB_ETIMEOUT;
-    }
-    return TB_OK;
 }
