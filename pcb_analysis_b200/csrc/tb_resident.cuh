@@ -182,6 +182,40 @@ __device__ __forceinline__ bool res_take(At&& at, unsigned int tag, int polls, f
     }
 }
 
+// Words of 48 bits of an FP64 value (rounded to 37 bits) and the tag's low 16:
+// enough to tell a word from the iteration before, the only older one it can
+// hold.  The blocks' parts of a patch sum keep more than FP32 on the way to
+// their sum, which alone is rounded to FP32.
+__device__ __forceinline__ void res_post48(unsigned long long* w, unsigned int tag, double v) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(v) + 0x8000ull;
+    const unsigned long long word = (bits & ~0xffffull) | (tag & 0xffffu);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(w), "l"(word) : "memory");
+}
+// The words at(0) .. at(N-1) (null: reads as 0), as res_take.
+template <int N, class At>
+__device__ __forceinline__ bool res_take48(At&& at, unsigned int tag, int polls, double (&v)[N]) {
+    const unsigned int mark = tag & 0xffffu;
+    unsigned long long word[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const unsigned long long* const w = at(k);
+        word[k] = w != nullptr ? res_peek(w) : (unsigned long long)mark;
+    }
+    for (int i = 0;; ++i) {
+        bool all = true;
+#pragma unroll
+        for (int k = 0; k < N; ++k) all = all && ((unsigned int)word[k] & 0xffffu) == mark;
+        if (all || i >= polls) {
+#pragma unroll
+            for (int k = 0; k < N; ++k) v[k] = __longlong_as_double((long long)(word[k] & ~0xffffull));
+            return all;
+        }
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            if (((unsigned int)word[k] & 0xffffu) != mark) word[k] = res_peek(at(k));
+    }
+}
+
 // A pair of words side by side (16 bytes, each word with its own tag).
 __device__ __forceinline__ void res_post2(unsigned long long* w, unsigned int tag, float a, float b) {
     const unsigned long long t = (unsigned long long)tag << 32;
@@ -471,8 +505,8 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_pcg(const __grid_cons
             if (TL && own[k]) s_res[t + k * kResThreads] = patch[k] >= 0 ? r[k] : 0.f;
         }
         if (TL) {
-            // sums of the block's part of each patch it touches: 16 lanes per
-            // patch, in FP32 per lane and FP64 across them
+            // sums of the block's part of each patch it touches, in FP64: 16 lanes
+            // per patch
             __syncthreads();
             const int lane = t & 15, pairs = prow_count * P.cl.nbx;
             for (int w = t >> 4; w < (pairs + 1) / 2 * 2; w += kResThreads / 16) {
@@ -481,29 +515,28 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_pcg(const __grid_cons
                 const int z = pr / P.cl.nby, y0 = (pr - z * P.cl.nby) * P.cl.b, x0 = pc * P.cl.b;
                 const int bw = min(P.cl.b, P.lay.C + 1 - x0), bh = min(P.cl.b, P.lay.R + 1 - y0);
                 const int first = (z * (P.lay.R + 1) + y0) * Xp, origin = first + x0 - base;
-                float s = 0.f;  // lane: every fourth column of every fourth row
+                double v = 0.0;  // lane: every fourth column of every fourth row
                 for (int yy = lane >> 2; real && yy < bh; yy += 4)
                     for (int xx = lane & 3; xx < bw; xx += 4) {
                         const int at = origin + yy * Xp + xx;
-                        if (at >= 0 && at < P.chunk) s += s_res[at];
+                        if (at >= 0 && at < P.chunk) v += (double)s_res[at];
                     }
-                double v = (double)s;
 #pragma unroll
                 for (int off = 8; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off, 16);
                 if (real && lane == 0 && !res_muted<MUTE>(P, kResPatchSums))
-                    res_post(P.part + (size_t)(blk - first / P.chunk) * P.cl.ld + (size_t)pr * P.cl.nbx + pc, tag, (float)v);
+                    res_post48(P.part + (size_t)(blk - first / P.chunk) * P.cl.ld + (size_t)pr * P.cl.nbx + pc, tag, v);
             }
             // R of the tile's columns and rows
             double sum = 0.0;
             for (int s0 = 0; s0 < P.slots; s0 += 4) {
-                float v[4];
-                ok = res_take(
+                double v[4];
+                ok = res_take48(
                          [&](const int k) -> const unsigned long long* {
                              return s0 + k < nslots ? P.part + (size_t)(s0 + k) * P.cl.ld + entry : nullptr;
                          },
                          tag, P.polls, v) &&
                      ok;
-                sum += ((double)v[0] + (double)v[1]) + ((double)v[2] + (double)v[3]);
+                sum += (v[0] + v[1]) + (v[2] + v[3]);
             }
             if (t < P.tcols + P.trows) s_R[t] = (float)sum;
             if (!__syncthreads_and(ok)) {
