@@ -3,6 +3,11 @@
 
 constexpr int kResLimit = 512;      // iterations of one launch (a few milliseconds)
 constexpr int kResMinChunk = 128;   // nodes of a block at least
+// Longest node row: a block stages two rows beside its nodes on each of three
+// planes, word by word.  Microseconds per iteration with Jacobi, this kernel /
+// the graph-captured ones: 1 x 4000 x 12 elements 12.0 / 16.7, 1 x 5000 x 8 12.7 /
+// 16.8, 2 x 5000 x 8 17.1 / 16.9, 1 x 6000 x 12 18.3 / 17.8, 1 x 7000 x 8 19.7 / 16.9.
+constexpr int kResMaxRow = 4800;
 
 using ResidentKernel = void (*)(const ResidentParams);
 template <bool MUTE>
@@ -29,7 +34,7 @@ int resident_setup(tb_system* s) {
     const Layout& L = s->lay;
     const bool tl = s->precond == 1;
     if (s->physics != 0 || s->precond > 1 || s->sms > kResMaxBlocks) return TB_OK;
-    if (L.L > (long long)s->sms * kResThreads * kResNodes) return TB_OK;
+    if (L.L > (long long)s->sms * kResThreads * kResNodes || L.Xp > kResMaxRow) return TB_OK;
     int coop = 0;
     TB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
     if (!coop) return TB_OK;

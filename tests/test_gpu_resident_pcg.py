@@ -195,3 +195,12 @@ def test_a_refused_kernel_leaves_the_solve_to_the_graph_kernels(ns_local, precon
     assert out[0]["converged"]
     np.testing.assert_array_equal(out[0]["solution"], out[1]["solution"])
     assert out[0]["history"] == out[1]["history"]
+
+
+@pytest.mark.parametrize("cols, taken", [(4799, True), (4803, False), (7000, False)])
+def test_boards_with_long_rows_stay_on_the_graph_kernels(ns_local, cols, taken):
+    config = MPIRConfig(inner_relative_tolerance=1e-30, max_outer_iterations=1, max_inner_iterations=30)
+    one, graph = _both(ns_local, _board(ns_local, 2, 1, cols, False, False), "jacobi", config)
+    assert (one["launches"] < graph["launches"]) == taken
+    if not taken:
+        np.testing.assert_array_equal(one["solution"], graph["solution"])
