@@ -91,7 +91,7 @@ struct BatchInstance {
     // two-level preconditioner (twolevel != 0): coarse grid, FP32 inverse of
     // Z^T A Z (nc x nc), R = Z^T r and c = Minv R
     CoarseLayout cl;
-    int twolevel, coarse_items;  // coarse_items: blocks of kCoarseRows rows of Minv
+    int twolevel;
     const float* minv;
     float *rc, *cvec;
     Layout lay;
@@ -107,7 +107,8 @@ struct BatchSchedule {
     int tile64[kBatchMax + 1];
     int chunk[kBatchMax + 1];
     int patch[kBatchMax + 1];  // two-level boards: one item per patch (restriction)
-    int crow[kBatchMax + 1];   // two-level boards: one item per kCoarseRows rows of Minv
+    int crow[kBatchMax + 1];   // two-level boards: one item per crow_rows rows of Minv
+    int crow_rows;
     // FP32 operator tiles handed out one at a time: [0] next tile, [1] blocks
     // done; the last block of a launch sets both back to zero.  [2], [3]: the
     // same for the coarse kernel's items.
@@ -115,11 +116,6 @@ struct BatchSchedule {
 };
 
 enum { ITEMS_TILE32 = 0, ITEMS_TILE64 = 1, ITEMS_CHUNK = 2, ITEMS_PATCH = 3, ITEMS_CROW = 4 };
-// Rows of the coarse inverse per item, four a warp: an item stages R, takes a
-// ticket and merges its part of R.c, some 4 us beside 1 us per row of reading
-// (ten boards of 2,000 unknowns: 53 us with eight rows, one a warp, 47).
-constexpr int kCoarseRows = 32;
-
 __global__ void batch_set_schedule(BatchSchedule value, BatchSchedule* dst) {
     const int* src = reinterpret_cast<const int*>(&value);
     int* out = reinterpret_cast<int*>(dst);
@@ -206,8 +202,8 @@ __device__ __forceinline__ int board_running_or_starting(const BatchInstance* I)
 }
 
 // Board ticket: true in every thread of the block that finished the board's
-// last item.  Thread 0 must have stored the block's partial before the call;
-// only its writes are published (the other threads' are read by later kernels).
+// last item.  What the block's threads wrote before the call (its partial) can
+// be read by that block.
 __device__ __forceinline__ bool last_item(unsigned int* counter, int items, bool* flag) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -611,10 +607,24 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// Rows row0, row0 + kCoarseWarps, .. (N of them) of c = Minv R by one warp.
+constexpr int kCoarseWarps = 8;
+template <int N>
+__device__ __forceinline__ void batch_coarse_rows(const BatchInstance* __restrict__ I, const float* s_rc, int row0, int lane) {
+    const int nc = I->cl.nc, ld = I->cl.ld;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        const int row = row0 + u * kCoarseWarps;
+        if (row >= nc) break;
+        const float sum = coarse_row(I->minv + (long long)row * ld, s_rc, ld, lane);
+        if (lane == 0) I->cvec[row] = sum;
+    }
+}
+
 // c = Minv R over the row blocks of every such board; the coarse part R.c of
 // r.z is reduced per board and its last item finishes the scalars (start:
 // rz; iteration: beta, breakdown and the iteration limit).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * kCoarseWarps)
     batch_coarse(const BatchInstance* __restrict__ table, const BatchSchedule* __restrict__ sched) {
     extern __shared__ float s_rc[];
     __shared__ ItemMap m;
@@ -623,7 +633,7 @@ __global__ void __launch_bounds__(256)
     Acc32* const red = reinterpret_cast<Acc32*>(red_raw);
     __shared__ int s_t;
     enter_items<ITEMS_CROW>(table, sched, m, board_running_or_starting);
-    const int total = m.prefix[m.n];
+    const int total = m.prefix[m.n], rows = sched->crow_rows;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned int* const grab = const_cast<unsigned int*>(sched->grab) + 2;
     // items (rows of boards whose coarse grids differ in size) taken one at a
@@ -643,22 +653,30 @@ __global__ void __launch_bounds__(256)
         const int nc = I->cl.nc, ld = I->cl.ld;
         for (int i = threadIdx.x; i < ld; i += blockDim.x) s_rc[i] = I->rc[i];
         __syncthreads();
-        Acc32 acc[1];
-        for (int u = warp; u < kCoarseRows; u += blockDim.x >> 5) {
-            const int row = (t - m.prefix[k]) * kCoarseRows + u;
-            if (row >= nc) break;
-            const float sum = coarse_row(I->minv + (long long)row * ld, s_rc, ld, lane);
-            if (lane == 0) {
-                I->cvec[row] = sum;
-                acc[0].add_product(s_rc[row], sum);
-            }
-        }
-        block_merge<1>(acc, red);
-        const int lt = t - m.prefix[k];
-        if (threadIdx.x == 0) acc_store(I->partials + (size_t)lt * 4, acc[0]);
-        if (last_item(I->counter + 1, I->coarse_items, &s_last)) {
+        const int row0 = (t - m.prefix[k]) * rows + warp;
+        if (rows == 32) batch_coarse_rows<4>(I, s_rc, row0, lane);
+        else if (rows == 16) batch_coarse_rows<2>(I, s_rc, row0, lane);
+        else batch_coarse_rows<1>(I, s_rc, row0, lane);
+        // the last item forms R.c over all rows, in an order of its own, so that
+        // a board's bits do not depend on how many rows an item had
+        if (last_item(I->counter + 1, (nc + rows - 1) / rows, &s_last)) {
             Acc32 tot[1];
-            grid_merge<1>(I->partials, I->coarse_items, 4, tot, red, I->counter + 1);
+            constexpr int AHEAD = 8;  // loads in flight
+            for (int first = threadIdx.x; first < nc; first += AHEAD * blockDim.x) {
+                float c[AHEAD];
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    const int row = first + u * blockDim.x;
+                    c[u] = row < nc ? __ldcg(I->cvec + row) : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    const int row = first + u * blockDim.x;
+                    if (row < nc) tot[0].add_product(s_rc[row], c[u]);
+                }
+            }
+            block_merge<1>(tot, red);
+            if (threadIdx.x == 0) I->counter[1] = 0u;
             if (threadIdx.x == 0) {
                 SolveCtl* ctl = I->ctl;
                 const double rzn = ctl->rdr + tot[0].value();

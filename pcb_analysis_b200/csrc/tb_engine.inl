@@ -300,7 +300,7 @@ Layout layout_of(const tb_system_desc* d) {
     return L;
 }
 
-int board_items(const Layout& L, int nc, int* tiles32, int* gx32, int* tiles64, int* gx64, int* chunks) {
+int board_items(const Layout& L, int* tiles32, int* gx32, int* tiles64, int* gx64, int* chunks) {
     *gx32 = apply_grid_x(L.C);
     tiles32[0] = *gx32 * apply_grid_y(8, L.R);
     tiles32[1] = *gx32 * apply_grid_y(16, L.R);
@@ -308,8 +308,7 @@ int board_items(const Layout& L, int nc, int* tiles32, int* gx32, int* tiles64, 
     *gx64 = apply_grid_x(L.C);
     *tiles64 = *gx64 * apply_grid_y(tb_engine::rows64, L.R);
     *chunks = (int)((L.L / 4 + kBatchChunkQuads - 1) / kBatchChunkQuads);
-    const int coarse_items = (nc + kCoarseRows - 1) / kCoarseRows;
-    return std::max(std::max(std::max(tiles32[0], *tiles64), *chunks), coarse_items);
+    return std::max(std::max(tiles32[0], *tiles64), *chunks);
 }
 
 template <typename T>
@@ -317,6 +316,21 @@ T* carve(char*& cursor, size_t count) {
     T* p = reinterpret_cast<T*>(cursor);
     cursor += (sizeof(T) * count + 255) / 256 * 256;
     return p;
+}
+
+// Rows of the coarse inverses per item of the coarse kernel, from the rows of all
+// resident boards.  An item stages its board's R and takes a ticket, so it
+// wants several rows; a few boards' rows have to be spread over the device.
+// Milliseconds for a batch of boards of some 1,900 rows each, 8 / 16 / 32 rows
+// an item:
+//   2 boards      5 boards      10 boards     24 boards     64 boards
+//   220/232/260   304/314/342   495/498/509   663/642/648   1275/1215/1190
+// (32 for all, each item merging its part of R.c: 255, 357, 530, 665 and 1220.)
+// The lines lie between 10 and 24 boards and between 24 and 64.
+int coarse_rows_per_item(long long rows, int sms) {
+    int per = kCoarseWarps;
+    while (per < 4 * kCoarseWarps && rows > 24LL * per * sms) per *= 2;
+    return per;
 }
 
 int engine_build_schedule(tb_engine* e) {
@@ -330,6 +344,9 @@ int engine_build_schedule(tb_engine* e) {
         if (e->slots[slot] && !e->slots[slot]->reported) order.push_back(slot);
     std::stable_sort(order.begin(), order.end(),
                      [&](int a, int b) { return e->slots[a]->lay.S > e->slots[b]->lay.S; });
+    long long rows = 0;
+    for (const int slot : order) rows += e->slots[slot]->cl.nc;
+    s.crow_rows = coarse_rows_per_item(rows, e->sms);
     int n = 0;
     for (const int slot : order) {
         const EngineBoard* b = e->slots[slot];
@@ -338,7 +355,7 @@ int engine_build_schedule(tb_engine* e) {
         s.tile64[n + 1] = s.tile64[n] + b->inst.tiles64;
         s.chunk[n + 1] = s.chunk[n] + b->inst.chunks;
         s.patch[n + 1] = s.patch[n] + b->cl.nc;
-        s.crow[n + 1] = s.crow[n] + b->inst.coarse_items;
+        s.crow[n + 1] = s.crow[n] + cdiv(b->cl.nc, s.crow_rows);
         ++n;
     }
     s.n = n;
@@ -505,7 +522,7 @@ int engine_submit(tb_engine* e, const tb_system_desc* d, const double* rhs, cons
     if (e->precond) tmp.cl = coarse_layout(L, 0);
     const int nc = tmp.cl.nc;
     int tiles64 = 0, gx64 = 0, chunks = 0, gx32 = 0;
-    const int max_items = board_items(L, nc, tmp.tiles32, &gx32, &tiles64, &gx64, &chunks);
+    const int max_items = board_items(L, tmp.tiles32, &gx32, &tiles64, &gx64, &chunks);
     size_t resident = 0, transient = 0;
     board_bytes(L, max_items, nc, &resident, &transient);
     if (e->in_use + (long long)(resident + transient) > e->budget)
@@ -631,7 +648,6 @@ int engine_submit(tb_engine* e, const tb_system_desc* d, const double* rhs, cons
     I.chunks = chunks;
     I.cl = b->cl;
     I.twolevel = nc > 0 ? 1 : 0;
-    I.coarse_items = (nc + kCoarseRows - 1) / kCoarseRows;
     I.minv = minv32;
     I.rc = rc;
     I.cvec = cvec;
@@ -915,7 +931,7 @@ int tb_engine_footprint(const tb_system_desc* desc, int32_t preconditioner, int6
     const Layout L = layout_of(desc);
     const int nc = preconditioner == 1 ? coarse_layout(L, 0).nc : 0;
     int t32[3], gx32, t64, gx64, chunks;
-    const int items = board_items(L, nc, t32, &gx32, &t64, &gx64, &chunks);
+    const int items = board_items(L, t32, &gx32, &t64, &gx64, &chunks);
     size_t r = 0, t = 0;
     board_bytes(L, items, nc, &r, &t);
     if (resident) *resident = (int64_t)r;

@@ -281,3 +281,20 @@ def test_tensor_copy_staging_across_boards_of_different_slab_counts() -> None:
         assert staged["converged"] and staged["relative_residual"] <= 1e-10
         np.testing.assert_array_equal(staged["solution"], plain["solution"])
         assert staged["inner_iterations"] == plain["inner_iterations"]
+
+
+def test_two_level_bits_do_not_depend_on_the_rows_an_item_has() -> None:
+    """Alone, among 16 and among 32 boards of some 2,000 coarse unknowns: the coarse
+    product is dealt out by 8, 16 and 32 rows."""
+
+    from pcb_analysis_b200._native import BatchEngine
+
+    boards = [_board(60 + i, 8, 55, 56, fixed=0.02) for i in range(32)]
+    results = []
+    with BatchEngine(capacity=32, max_slabs=8, tile_rows=16, preconditioner="two-level", staging="cp.async") as engine:
+        for count in (1, 16, 32):
+            tickets = [engine.submit(arrays, rhs, CONFIG) for arrays, rhs in boards[:count]]
+            results.append(_drain(engine, count)[tickets[0]])
+    for other in results[1:]:
+        np.testing.assert_array_equal(other["solution"], results[0]["solution"])
+        assert other["history"] == results[0]["history"]
