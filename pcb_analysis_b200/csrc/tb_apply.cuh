@@ -113,6 +113,15 @@ __device__ __forceinline__ Quad<double> ldg_quad(const double* p) {
     const double2 b = __ldg(reinterpret_cast<const double2*>(p) + 1);
     return {{a.x, a.y, b.x, b.y}};
 }
+// The same of an operand that the kernel before wrote (no read-only load).
+__device__ __forceinline__ Quad<float> ld_quad(const float* p) {
+    const float4 a = *reinterpret_cast<const float4*>(p);
+    return {{a.x, a.y, a.z, a.w}};
+}
+__device__ __forceinline__ Quad<double> ld_quad(const double* p) {
+    const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+    return {{a.x, a.y, b.x, b.y}};
+}
 __device__ __forceinline__ void st_quad(float* p, const Quad<float>& q) {
     *reinterpret_cast<float4*>(p) = make_float4(q.v[0], q.v[1], q.v[2], q.v[3]);
 }

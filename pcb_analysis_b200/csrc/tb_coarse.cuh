@@ -70,7 +70,7 @@ __global__ void coarse_indicator(double* __restrict__ x, const double* __restric
 // per-iteration restriction of the inner PCG (the precision the reference's
 // low-precision runtime uses for it), FP64 for the set-up.
 template <typename T>
-__device__ __forceinline__ T patch_sum(const T* __restrict__ v, const T* __restrict__ mask, long long base, int bh,
+__device__ __forceinline__ T patch_sum(const T* v, const T* __restrict__ mask, long long base, int bh,
                                        int bw, int Xp) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     T acc = T(0);
@@ -97,7 +97,7 @@ __device__ __forceinline__ T patch_sum(const T* __restrict__ v, const T* __restr
 // solve state, the whole grid returns unless the PCG is running.
 template <typename T>
 __global__ void __launch_bounds__(128)
-    coarse_restrict(const T* __restrict__ v, const T* __restrict__ mask, T* __restrict__ out, Layout lay,
+    coarse_restrict(const T* v, const T* __restrict__ mask, T* __restrict__ out, Layout lay,
                     CoarseLayout cl, long long pstride, const SolveCtl* ctl) {
     __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc64) * 32];
     Acc64* const scratch = reinterpret_cast<Acc64*>(scratch_raw);
@@ -476,7 +476,7 @@ constexpr int kCoarseThreads = 1024;  // R is staged once per block for 8 rows a
 // there); four warps per row keep enough loads in flight to cover its latency.
 template <int MODE>
 __global__ void __launch_bounds__(kCoarseThreads, 2)
-    coarse_apply(const float* __restrict__ minv, const float* __restrict__ rc, float* __restrict__ c, int nc, int ld,
+    coarse_apply(const float* __restrict__ minv, const float* rc, float* __restrict__ c, int nc, int ld,
                  SolveCtl* ctl, double* partials, unsigned int* counter) {
     extern __shared__ float s_rc[];
     __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc32) * 32];
@@ -526,8 +526,8 @@ __global__ void __launch_bounds__(kCoarseThreads, 2)
 // Not START: x += alpha p first (the update's step, on the old p).
 template <bool START>
 __global__ void __launch_bounds__(kVecThreads)
-    pcg_direction_2l(float* __restrict__ p, float* __restrict__ x, const float* __restrict__ r,
-                     const float* __restrict__ dinv, const float* __restrict__ c, long long nq, Layout lay,
+    pcg_direction_2l(float* __restrict__ p, float* __restrict__ x, const float* r,
+                     const float* __restrict__ dinv, const float* c, long long nq, Layout lay,
                      CoarseLayout cl, const SolveCtl* ctl) {
     pdl_enter();
     if (ctl != nullptr && ctl->state != ST_RUNNING) return;

@@ -119,9 +119,9 @@ __device__ __forceinline__ DcRow<T> dc_load_row(const DcParams<T>& P, const int 
     r.m = make_uchar4(0, 0, 0, 0);
     r.right = T(0);
     if (quad_ok && yy >= 0 && yy <= R) {
-        r.raw = ldg_quad(P.A.x + n);
+        r.raw = ld_quad(P.A.x + n);
         r.m = *reinterpret_cast<const uchar4*>(P.mask + n);
-        if (edge_ok) r.right = dc_masked(__ldg(P.A.x + n + 4), P.mask[n + 4], STIFF);
+        if (edge_ok) r.right = dc_masked(P.A.x[n + 4], P.mask[n + 4], STIFF);
     }
     r.w[0] = dc_masked(r.raw.v[0], r.m.x, STIFF);
     r.w[1] = dc_masked(r.raw.v[1], r.m.y, STIFF);

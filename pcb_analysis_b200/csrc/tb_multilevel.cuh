@@ -35,6 +35,11 @@
 // level's pre-smoothing), the dense coarse product, per level ml_up (the
 // prolonged residual and the post-smoothing; the top one finishes r.z and
 // beta), and ml_direction (p = T^-1 r + Z_1 c + beta p, x += alpha p).
+//
+// The kernels of an iteration are programmatic dependents of one another: an
+// operand that one of them writes is neither const __restrict__ nor read by
+// __ldg in the others, since a read-only load may be taken for independent of
+// the dependency wait.  Coefficients and factors, written at set-up only, are.
 #pragma once
 
 #include <cuda.h>  // CUtensorMap (the type only; maps are encoded by the host)
@@ -100,7 +105,7 @@ __device__ __forceinline__ T ml_coef(const T* __restrict__ st, long long n, long
 // Indices are 32-bit: a level's 14 stencil arrays hold fewer than 2^31
 // values (checked at set-up).
 template <bool INTERIOR>
-__device__ __forceinline__ float ml_stencil_dot(const float* __restrict__ st, const float* __restrict__ v,
+__device__ __forceinline__ float ml_stencil_dot(const float* __restrict__ st, const float* v,
                                                 const MLGrid& g, int z, int y, int x) {
     const int n = (int)g.n, plane = (int)g.plane, nx = g.nx;
     const int i = z * plane + y * nx + x;
@@ -117,7 +122,7 @@ __device__ __forceinline__ float ml_stencil_dot(const float* __restrict__ st, co
                 const int o = (dz + 1) * 9 + (dy + 1) * 3 + (dx + 1);
                 const int j = i + dz * plane + dy * nx + dx;
                 const float a = (o >= 13) ? __ldg(st + (o - 13) * n + i) : __ldg(st + (13 - o) * n + j);
-                acc = fmaf(a, __ldg(v + j), acc);
+                acc = fmaf(a, v[j], acc);
             }
         }
     }
@@ -228,7 +233,7 @@ struct MLPre {
 // reciprocal (their block row is the identity, so w = r there); pads carry 0.
 template <int NP, int MODE>
 __global__ void __launch_bounds__(kMlThreads)
-    ml_update(float* __restrict__ r, const float* __restrict__ q, const double* __restrict__ r64,
+    ml_update(float* __restrict__ r, const float* q, const double* r64,
               float* __restrict__ x32, float* __restrict__ w, float* __restrict__ R1, const float* __restrict__ zl,
               const float* __restrict__ zi, Layout lay, long long pstride, MLGrid g1, MLNext nx, SolveCtl* ctl,
               double* partials, unsigned int* counter, KernelClock* clock) {
@@ -500,8 +505,8 @@ __global__ void __launch_bounds__(kMlThreads, 1)
 // x += alpha p, r -= alpha q, r.r (FP64); the stopping test; r.z and beta
 // follow from the preconditioner's kernels.
 __global__ void __launch_bounds__(kVecThreads)
-    pcg_update_f64_norm(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ p,
-                        const double* __restrict__ q, long long nq, SolveCtl* ctl, double* partials,
+    pcg_update_f64_norm(double* __restrict__ x, double* __restrict__ r, const double* p,
+                        const double* q, long long nq, SolveCtl* ctl, double* partials,
                         unsigned int* counter) {
     __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc64) * 32];
     Acc64* const scratch = reinterpret_cast<Acc64*>(scratch_raw);
@@ -531,7 +536,7 @@ __global__ void __launch_bounds__(kVecThreads)
 // p = f64(T^-1 r + Z_1 c) + beta p (START: without beta p).
 template <bool START>
 __global__ void __launch_bounds__(kVecThreads)
-    ml_direction_f64(double* __restrict__ p, const float* __restrict__ w, const float* __restrict__ c1,
+    ml_direction_f64(double* __restrict__ p, const float* w, const float* c1,
                      const float* __restrict__ zi, long long nq, Layout lay, MLGrid g1,
                      unsigned long long fixed_planes, const SolveCtl* ctl) {
     pdl_enter();
@@ -575,8 +580,8 @@ __global__ void __launch_bounds__(kVecThreads)
 // reciprocal) is read only on planes that hold a fixed node.
 template <bool START>
 __global__ void __launch_bounds__(kVecThreads)
-    ml_direction(float* __restrict__ p, float* __restrict__ x, const float* __restrict__ w,
-                 const float* __restrict__ c1, const float* __restrict__ zi, long long nq, Layout lay, MLGrid g1,
+    ml_direction(float* __restrict__ p, float* __restrict__ x, const float* w,
+                 const float* c1, const float* __restrict__ zi, long long nq, Layout lay, MLGrid g1,
                  unsigned long long fixed_planes, const SolveCtl* ctl) {
     pdl_enter();
     if (ctl != nullptr && ctl->state != ST_RUNNING) return;
@@ -679,7 +684,7 @@ __device__ __forceinline__ void ml_load_stencil(float (&a)[27], const float* __r
         a[o] = in ? __ldg(o >= 13 ? st + (o - 13) * n + i : st + (13 - o) * n + j) : 0.f;
     }
 }
-__device__ __forceinline__ float ml_stencil_dot_held(const float (&a)[27], const float* __restrict__ v,
+__device__ __forceinline__ float ml_stencil_dot_held(const float (&a)[27], const float* v,
                                                      const MLGrid& g, int z, int y, int x) {
     float acc = 0.f;
 #pragma unroll
@@ -914,7 +919,7 @@ constexpr int kMlWideThreads = kMlWideX * kMlWideY;
 
 template <int NP, int B>
 __global__ void __launch_bounds__(kMlWideThreads, 4)
-    ml_down_wide(const float* __restrict__ st, const float* __restrict__ R, const float* __restrict__ xv,
+    ml_down_wide(const float* __restrict__ st, const float* R, const float* xv,
                  const float* __restrict__ ipd, float* __restrict__ sv, float* __restrict__ Rc, float* xc,
                  const float* __restrict__ lfc, const float* __restrict__ ipdc, MLGrid g, MLGrid gc,
                  const SolveCtl* ctl) {
@@ -1020,8 +1025,8 @@ __global__ void __launch_bounds__(kMlWideThreads, 4)
 
 template <int NP, int B, bool TOP>
 __global__ void __launch_bounds__(kMlWideThreads, NP <= 18 ? 4 : 3)
-    ml_up_wide(const float* __restrict__ az, const float* __restrict__ R, const float* __restrict__ sv,
-               const float* __restrict__ xv, const float* __restrict__ cn, const float* __restrict__ lf,
+    ml_up_wide(const float* __restrict__ az, const float* R, const float* sv,
+               const float* xv, const float* cn, const float* __restrict__ lf,
                const float* __restrict__ ipd, float* __restrict__ yo, MLGrid g, MLGrid gc, SolveCtl* ctl,
                int mode, double* partials, unsigned int* counter) {
     __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc32) * 32];
@@ -1113,7 +1118,7 @@ __global__ void __launch_bounds__(kMlWideThreads, NP <= 18 ? 4 : 3)
 // per thread (see MLPre).
 template <int NP>
 __global__ void __launch_bounds__(kMlWideThreads)
-    ml_presmooth(const float* __restrict__ R, float* __restrict__ xo, const float* __restrict__ lf,
+    ml_presmooth(const float* R, float* __restrict__ xo, const float* __restrict__ lf,
                  const float* __restrict__ ipd, MLGrid g, const SolveCtl* ctl) {
     pdl_enter();
     if (ctl != nullptr && ctl->state != ST_RUNNING) return;

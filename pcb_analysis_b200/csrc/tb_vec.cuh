@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kPackThreads)
 // set, src is incomplete and dst is left as it is.
 template <int LANES, typename T>
 __global__ void __launch_bounds__(kPackThreads)
-    unpack_nodes(T* __restrict__ dst, const T* __restrict__ src, Layout lay, PackShape p, const int* err) {
+    unpack_nodes(T* __restrict__ dst, const T* src, Layout lay, PackShape p, const int* err) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (err != nullptr && *err != 0) return;
@@ -95,8 +95,15 @@ __global__ void __launch_bounds__(kPackThreads)
         const T* const s = src + line * lay.Xp;
         T* const d = dst + line * cols;
         const int end = min(x1, cols);
-#pragma unroll 4
-        for (int x = x0 + lane; x < end; x += LANES) d[x] = s[x];
+        int x = x0 + lane;
+        for (; x + 3 * LANES < end; x += 4 * LANES) {  // four loads in flight
+            T v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = s[x + u * LANES];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) d[x + u * LANES] = v[u];
+        }
+        for (; x < end; x += LANES) d[x] = s[x];
     });
 }
 
@@ -408,7 +415,7 @@ __device__ __forceinline__ bool x_step_pending(const SolveCtl* c) {
 // less traffic.
 template <bool TL>
 __global__ void __launch_bounds__(kVecThreads)
-    pcg_update_f32(float* __restrict__ r, const float* __restrict__ q, const float* __restrict__ dinv, long long nq,
+    pcg_update_f32(float* __restrict__ r, const float* q, const float* __restrict__ dinv, long long nq,
                    SolveCtl* ctl, double* partials, unsigned int* counter) {
     __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc32) * (2 * 32)];
     Acc32* const scratch = reinterpret_cast<Acc32*>(scratch_raw);
@@ -444,8 +451,8 @@ __global__ void __launch_bounds__(kVecThreads)
 }
 
 __global__ void __launch_bounds__(kVecThreads)
-    pcg_update_f64(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ p,
-                   const double* __restrict__ q, const double* __restrict__ dinv, long long nq, SolveCtl* ctl,
+    pcg_update_f64(double* __restrict__ x, double* __restrict__ r, const double* p,
+                   const double* q, const double* __restrict__ dinv, long long nq, SolveCtl* ctl,
                    double* partials, unsigned int* counter) {
     __shared__ __align__(16) unsigned char scratch_raw[sizeof(Acc64) * (2 * 32)];
     Acc64* const scratch = reinterpret_cast<Acc64*>(scratch_raw);
@@ -479,7 +486,7 @@ __global__ void __launch_bounds__(kVecThreads)
 // x += alpha p (the update's step, on the old p), then p = z + beta p with
 // z = r / d (reference solver.py:199-224).
 __global__ void __launch_bounds__(kVecThreads)
-    pcg_direction_f32(float* __restrict__ p, float* __restrict__ x, const float* __restrict__ r,
+    pcg_direction_f32(float* __restrict__ p, float* __restrict__ x, const float* r,
                       const float* __restrict__ dinv, long long nq, const SolveCtl* ctl) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -506,7 +513,7 @@ __global__ void __launch_bounds__(kVecThreads)
 }
 
 __global__ void __launch_bounds__(kVecThreads)
-    pcg_direction_f64(double* __restrict__ p, const double* __restrict__ r, const double* __restrict__ dinv,
+    pcg_direction_f64(double* __restrict__ p, const double* r, const double* __restrict__ dinv,
                       long long nq, const SolveCtl* ctl) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

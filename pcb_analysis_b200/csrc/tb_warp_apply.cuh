@@ -130,9 +130,9 @@ __global__ void __launch_bounds__(32 * kWarpBlockWarps, 4) warp_apply_kernel(con
         for (int k = 0; k < NP; ++k) {
             const int off = k * pstride + rowoff;
             const bool ok = row_ok && plane_ok[k] && node_col_ok;
-            xa[k] = ok ? __ldg(xbase + off) : 0.0f;
+            xa[k] = ok ? xbase[off] : 0.0f;
             const bool rok = row_ok && plane_ok[k] && right_col_ok && edge;
-            xra[k] = rok ? __ldg(xbase + off + 1) : 0.0f;
+            xra[k] = rok ? xbase[off + 1] : 0.0f;
         }
         const int hi = S * pstride + rowoff;
         ra_lo = (has_lo && row_ok && node_col_ok) ? __ldg(rbase + rowoff) : 0.0f;
