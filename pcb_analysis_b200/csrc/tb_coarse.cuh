@@ -155,39 +155,6 @@ __global__ void coarse_fix_empty(double* __restrict__ M, const double* __restric
     }
 }
 
-// Gauss-Jordan step k, part 1: copy row k and column k; flag a pivot that is
-// not positive and finite.
-__global__ void gj_pivot(const double* __restrict__ A, double* __restrict__ rk, double* __restrict__ ck, int nc, int k,
-                         int* err) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nc; j += gridDim.x * blockDim.x) {
-        rk[j] = A[(long long)k * nc + j];
-        ck[j] = A[(long long)j * nc + k];
-        if (j == k) {
-            const double piv = A[(long long)k * nc + k];
-            if (!(piv > 0.0) || !isfinite(piv)) atomicOr(err, 1);
-        }
-    }
-}
-
-// Part 2: eliminate with pivot k in place (rows and columns k become the
-// inverse's).
-__global__ void gj_update(double* __restrict__ A, const double* __restrict__ rk, const double* __restrict__ ck, int nc,
-                          int k) {
-    const double p = 1.0 / ck[k];
-    const long long total = (long long)nc * nc;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
-        const int i = (int)(e / nc);
-        const int j = (int)(e - (long long)i * nc);
-        double v;
-        if (i == k && j == k) v = p;
-        else if (i == k) v = rk[j] * p;
-        else if (j == k) v = -ck[i] * p;
-        else v = A[e] - ck[i] * (rk[j] * p);
-        A[e] = v;
-    }
-}
-
 // ---- blocked Gauss-Jordan inversion (no pivoting; the matrix is SPD).
 // With A split in kGjB x kGjB blocks, block step K is
 //     P = A_KK^-1,  A_KJ <- P A_KJ,  A_IJ <- A_IJ - A_IK A_KJ,  A_IK <- -A_IK P,  A_KK <- P

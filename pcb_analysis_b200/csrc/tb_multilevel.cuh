@@ -916,14 +916,15 @@ __global__ void __launch_bounds__(kMlCols* kMlMaxGroups)
 // bytes a node; ml_down_wide 120, now 108: 3.1 TB/s).
 constexpr int kMlWideX = 32, kMlWideY = 4;  // columns of a block of ml_down_wide
 constexpr int kMlWideThreads = kMlWideX * kMlWideY;
+constexpr int kMlWideAgg = 2;  // a level with 4 x 4 aggregates is never wide: 200 x 200 columns at most
 
-template <int NP, int B>
+template <int NP>
 __global__ void __launch_bounds__(kMlWideThreads, 4)
     ml_down_wide(const float* __restrict__ st, const float* R, const float* xv,
                  const float* __restrict__ ipd, float* __restrict__ sv, float* __restrict__ Rc, float* xc,
                  const float* __restrict__ lfc, const float* __restrict__ ipdc, MLGrid g, MLGrid gc,
                  const SolveCtl* ctl) {
-    constexpr int CX = kMlWideX / B, CY = kMlWideY / B, CC = CX * CY;  // coarse columns of the block
+    constexpr int B = kMlWideAgg, CX = kMlWideX / B, CY = kMlWideY / B, CC = CX * CY;  // coarse columns of the block
     __shared__ float s_part[NP][kMlWideY][CX];  // per node row: sums over the row's part of an aggregate
     __shared__ float s_r[NP][CC], s_lf[NP][CC], s_ip[NP][CC];
     const int t = threadIdx.x, lane = t & 31, row = t >> 5;
@@ -999,15 +1000,13 @@ __global__ void __launch_bounds__(kMlWideThreads, 4)
                 if (!(pc >= 0.f)) v = 0.f;
             }
             v += __shfl_xor_sync(0xffffffffu, v, 1);
-            if (B == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
             if ((lane & (B - 1)) == 0) s_part[z][row][lane / B] = v;
         }
     }
     __syncthreads();
     for (int e = t; e < g.L * CC; e += kMlWideThreads) {
         const int z = e / CC, c = e % CC, w0 = (c / CX) * B;
-        float sum = s_part[z][w0][c % CX] + s_part[z][w0 + 1][c % CX];
-        if (B == 4) sum += s_part[z][(w0 + 2) % kMlWideY][c % CX] + s_part[z][(w0 + 3) % kMlWideY][c % CX];
+        const float sum = s_part[z][w0][c % CX] + s_part[z][w0 + 1][c % CX];
         const int AX = blockIdx.x * CX + c % CX, AY = blockIdx.y * CY + c / CX;
         if (AX < gc.nx && AY < gc.ny) Rc[ml_index(gc, z, AY, AX)] = sum;
         s_r[z][c] = sum;
@@ -1023,7 +1022,7 @@ __global__ void __launch_bounds__(kMlWideThreads, 4)
     }
 }
 
-template <int NP, int B, bool TOP>
+template <int NP, bool TOP>
 __global__ void __launch_bounds__(kMlWideThreads, NP <= 18 ? 4 : 3)
     ml_up_wide(const float* __restrict__ az, const float* R, const float* sv,
                const float* xv, const float* cn, const float* __restrict__ lf,
@@ -1036,6 +1035,7 @@ __global__ void __launch_bounds__(kMlWideThreads, NP <= 18 ? 4 : 3)
     const bool mine = c < plane;
     const int cl = mine ? c : plane - 1;  // clamped: valid addresses, results unused
     const int y = cl / g.nx, x = cl - y * g.nx;
+    constexpr int B = kMlWideAgg;
     const int Y = y / B, X = x / B;
     const int Ys = min(max(Y + ((y - Y * B < B / 2) ? -1 : 1), 0), gc.ny - 1);
     const int Xs = min(max(X + ((x - X * B < B / 2) ? -1 : 1), 0), gc.nx - 1);

@@ -148,12 +148,14 @@ cudaError_t ml_launch_down(tb_system* s, int l, bool pdl, const SolveCtl* ctl) {
     const tb_system::MLLevel& dn = s->ml[l + 1];
     const bool dense = l + 2 == (int)s->ml.size();
     const dim3 grid = ml_level_grid(lv.g);
-    if (ml_wide_down(s, lv.g)) {
-        constexpr int NP = ROUNDS == 1 ? 9 : (ROUNDS == 2 ? 18 : 33);
-        return ml_launch(pdl, ml_down_wide<NP, B>, dim3(ml_cdiv(lv.g.nx, kMlWideX), ml_cdiv(lv.g.ny, kMlWideY)),
-                         dim3(kMlWideThreads), s->stream, (const float*)lv.st, (const float*)lv.R, (const float*)lv.x,
-                         (const float*)lv.ipd, lv.s, dn.R, dense ? (float*)nullptr : dn.x, (const float*)dn.lf,
-                         (const float*)dn.ipd, lv.g, dn.g, ctl);
+    if constexpr (B == kMlWideAgg) {
+        if (ml_wide_down(s, lv.g)) {
+            constexpr int NP = ROUNDS == 1 ? 9 : (ROUNDS == 2 ? 18 : 33);
+            return ml_launch(pdl, ml_down_wide<NP>, dim3(ml_cdiv(lv.g.nx, kMlWideX), ml_cdiv(lv.g.ny, kMlWideY)),
+                             dim3(kMlWideThreads), s->stream, (const float*)lv.st, (const float*)lv.R,
+                             (const float*)lv.x, (const float*)lv.ipd, lv.s, dn.R, dense ? (float*)nullptr : dn.x,
+                             (const float*)dn.lf, (const float*)dn.ipd, lv.g, dn.g, ctl);
+        }
     }
     const bool pre = CAN && (int)(grid.x * grid.y) <= kMlPreBlocks * s->sms;
     return ml_launch_smem(pdl, pre ? ml_down<B, ROUNDS, CAN> : ml_down<B, ROUNDS, false>, grid,
@@ -176,13 +178,14 @@ cudaError_t ml_launch_up(tb_system* s, int l, int mode, bool pdl) {
     const tb_system::MLLevel& lv = s->ml[l];
     const tb_system::MLLevel& dn = s->ml[l + 1];
     SolveCtl* const state = mode == ML_ONLY ? nullptr : s->ctl;
-    if (ml_wide_up(s, lv.g)) {
-        constexpr int NP = ROUNDS == 1 ? 9 : (ROUNDS == 2 ? 18 : 33);
-        return ml_launch(pdl, l == 0 ? ml_up_wide<NP, B, true> : ml_up_wide<NP, B, false>,
-                         ml_column_grid(lv.g), dim3(kMlWideThreads), s->stream, (const float*)lv.az,
-                         (const float*)lv.R, (const float*)lv.s, (const float*)lv.x, (const float*)dn.y,
-                         (const float*)lv.lf, (const float*)lv.ipd, lv.y, lv.g, dn.g, state, mode,
-                         s->partials, s->counter);
+    if constexpr (B == kMlWideAgg) {
+        if (ml_wide_up(s, lv.g)) {
+            constexpr int NP = ROUNDS == 1 ? 9 : (ROUNDS == 2 ? 18 : 33);
+            return ml_launch(pdl, l == 0 ? ml_up_wide<NP, true> : ml_up_wide<NP, false>, ml_column_grid(lv.g),
+                             dim3(kMlWideThreads), s->stream, (const float*)lv.az, (const float*)lv.R,
+                             (const float*)lv.s, (const float*)lv.x, (const float*)dn.y, (const float*)lv.lf,
+                             (const float*)lv.ipd, lv.y, lv.g, dn.g, state, mode, s->partials, s->counter);
+        }
     }
     return ml_launch_smem(pdl, l == 0 ? ml_up<B, ROUNDS, true> : ml_up<B, ROUNDS, false>,
                           ml_level_grid(lv.g), dim3(kMlCols * ml_level_groups(lv.g.L)), ml_level_smem(lv.g.L),
