@@ -204,3 +204,84 @@ def test_boards_with_long_rows_stay_on_the_graph_kernels(ns_local, cols, taken):
     assert (one["launches"] < graph["launches"]) == taken
     if not taken:
         np.testing.assert_array_equal(one["solution"], graph["solution"])
+
+
+def _rows(mesh):
+    """The operator's rows in FP64: couplings [27, nodes] in the order (dz, dy, dx)
+    ascending, the centre left out."""
+
+    a = np.zeros((27,) + mesh.node_shape)
+    parts = [c.reshape(mesh.conductivity_w_per_m_k.shape) for c in mesh.element_coefficients()]
+    slabs, rows, cols = parts[0].shape
+    ends = [(o, b) for o in np.ndindex(2, 2, 2) for b in np.ndindex(2, 2, 2) if b != (0, 0, 0)]
+    for corner, other in ends:
+        m = [1.0 / 6.0 if t else 2.0 / 6.0 for t in other]
+        s = [-1.0 if t else 1.0 for t in other]
+        k = parts[0] * (m[0] * m[1] * s[2]) + parts[1] * (m[0] * s[1] * m[2]) + parts[2] * (s[0] * m[1] * m[2])
+        step = [(1 - 2 * c) * t for c, t in zip(corner, other)]
+        o = (step[0] + 1) * 9 + (step[1] + 1) * 3 + step[2] + 1
+        a[o][corner[0] : corner[0] + slabs, corner[1] : corner[1] + rows, corner[2] : corner[2] + cols] += k
+    return a
+
+
+@pytest.mark.parametrize(
+    "slabs, rows, cols, fixed, void",
+    [(8, 37, 44, True, True), (16, 30, 41, False, False), (16, 80, 100, True, False), (3, 210, 19, False, True)],
+)
+@pytest.mark.parametrize("smooth", [False, True])
+def test_two_iterations_match_fp64(ns_local, slabs, rows, cols, fixed, void, smooth):
+    """Two inner iterations against the same in FP64, node by node.
+
+    The second direction holds the first action of the kernel's own operator at
+    every node, so a wrong coefficient shows where it stands.  Bound: the
+    magnitudes that a node's value is made of (the action's taken on differences,
+    as the kernel does) times 32 units of FP32 rounding: some 24 roundings of half
+    a unit each along the way, and as much again for the scalars."""
+
+    problem = _board(ns_local, slabs, rows, cols, fixed, void)
+    op = ns_local.MatrixFreeThermalOperator(problem, preconditioner="jacobi")
+    config = MPIRConfig(inner_relative_tolerance=1e-30, max_outer_iterations=1, max_inner_iterations=2)
+    try:
+        shape = problem.mesh.node_shape
+        free = op.free_nodes.reshape(-1)
+        d = op.diagonal_high().reshape(-1)
+        rng = np.random.default_rng(slabs + rows)
+        v = rng.standard_normal(shape)
+        if smooth:  # nearly constant through the stack
+            v = v[:1] + 1e-3 * v
+        r0 = d * v.reshape(-1) * free
+        got = op.device_system.solve_mpir(r0, config)["solution"]
+        action = op.apply_high
+        p0 = r0 / d
+        q0 = action(p0)
+        rz0 = r0 @ p0
+        a0 = rz0 / (p0 @ q0)
+        r1 = r0 - a0 * q0
+        z1 = r1 / d
+        b0 = (r1 @ z1) / rz0
+        p1 = z1 + b0 * p0
+        a1 = (r1 @ z1) / (p1 @ action(p1))
+    finally:
+        op.close()
+    expected = a0 * p0 + a1 * p1
+    rows27 = _rows(problem.mesh)
+    u = np.pad((p0 * free).reshape(shape), 1)
+    centre = p0.reshape(shape)
+    size = np.zeros(shape)
+    view = lambda dz, dy, dx: u[1 + dz : u.shape[0] - 1 + dz, 1 + dy : u.shape[1] - 1 + dy, 1 + dx : u.shape[2] - 1 + dx]
+    total = np.zeros(shape)
+    for dy in (-1, 0, 1):
+        for dx in (-1, 0, 1):
+            k = (dy + 1) * 3 + dx + 1
+            low, mid, high = rows27[k], rows27[9 + k], rows27[18 + k]
+            side = view(0, dy, dx)
+            size += np.abs(low * (view(-1, dy, dx) - side)) + np.abs(high * (view(1, dy, dx) - side))
+            size += np.abs((low + mid + high) * (side - centre))
+            total += low + mid + high
+    robin = np.maximum(d.reshape(shape) + total, 0.0)  # the diagonal less the element part: R
+    size += robin * np.abs(centre)
+    size = size.reshape(-1)
+    bound = np.abs(a0 * p0) + np.abs(a1) * ((np.abs(r0) + np.abs(a0) * size) / d + np.abs(b0 * p0))
+    eps = np.finfo(np.float32).eps
+    assert np.all(np.abs(got - expected)[free] <= 32 * eps * bound[free])
+    assert np.linalg.norm((got - expected)[free]) <= 8 * eps * np.linalg.norm(bound[free])
