@@ -158,6 +158,7 @@ int engine_kernels_per_chunk(const tb_engine* e) { return 3 + (e->precond ? 5 : 
 
 void engine_free(tb_engine* e) {
     if (!e) return;
+    engine_idle(e);
     cudaSetDevice(e->device);
     if (e->stream) cudaStreamSynchronize(e->stream);
     if (e->io) cudaStreamSynchronize(e->io);
@@ -790,6 +791,7 @@ int engine_retire_oldest(tb_engine* e) {
     const int k = (e->head - e->inflight + kEngineDepth) % kEngineDepth;
     TB_CUDA(cudaEventSynchronize(e->ev[k]));
     e->inflight -= 1;
+    if (e->inflight == 0) engine_idle(e);
     const BatchStatus* snap = e->h_status + (size_t)k * e->capacity;
     for (int s = 0; s < e->capacity; ++s) {
         EngineBoard* b = e->slots[s];
@@ -820,6 +822,7 @@ int engine_step(tb_engine* e, int* finished) {
         TB_CUDA(cudaMemcpyAsync(e->h_status + (size_t)e->head * e->capacity, e->d_status,
                                 sizeof(BatchStatus) * e->capacity, cudaMemcpyDeviceToHost, e->stream));
         TB_CUDA(cudaEventRecord(e->ev[e->head], e->stream));
+        engine_queued(e, e->device, e->ev[e->head]);
         e->head = (e->head + 1) % kEngineDepth;
         e->inflight += 1;
     }

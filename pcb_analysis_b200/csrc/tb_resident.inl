@@ -2,6 +2,15 @@
 // Included by tb_system.cu inside its anonymous namespace.
 
 constexpr int kResLimit = 512;      // iterations of one launch (a few milliseconds)
+// The same beside a batch engine.  The kernel wants every SM, and gets in between
+// two of the engine's kernels: with launches of 512 iterations one after another a
+// thread of small solves left an engine a sixth of the device.  So each launch
+// waits for what the engine has queued, a chunk or two, and is short.  Ten boards'
+// batch (0.50 s alone) beside a thread of 96 x 80 x 8 two-level solves (0.029 s
+// alone): 3.1 s and 0.033 s a solve before; 0.93 and 0.11 with 128 iterations, 0.84
+// and 0.18 with 64, 0.70 and 0.30 with 32; 0.57 and 0.07 .. 0.20 with the
+// graph-captured kernels.
+constexpr int kResLimitShared = 64;
 constexpr int kResMinChunk = 128;   // nodes of a block at least
 // Longest node row: a block stages two rows beside its nodes on each of three
 // planes, word by word.  Microseconds per iteration with Jacobi, this kernel /
@@ -14,6 +23,37 @@ template <bool MUTE>
 ResidentKernel resident_kernel(int nodes, bool tl) {
     if (nodes == 1) return tl ? resident_pcg<1, true, MUTE> : resident_pcg<1, false, MUTE>;
     return tl ? resident_pcg<2, true, MUTE> : resident_pcg<2, false, MUTE>;
+}
+
+// The chunks that this process's batch engines have queued, by engine: the device
+// and the event behind the last one.  An engine is listed while any is in flight.
+struct EngineQueues {
+    std::mutex mu;
+    std::map<const void*, std::pair<int, cudaEvent_t>> busy;
+};
+EngineQueues& engine_queues() {
+    static EngineQueues* const q = new EngineQueues;  // outlives every engine
+    return *q;
+}
+void engine_queued(const void* engine, int device, cudaEvent_t last) {
+    std::lock_guard<std::mutex> lock(engine_queues().mu);
+    engine_queues().busy[engine] = {device, last};
+}
+void engine_idle(const void* engine) {
+    std::lock_guard<std::mutex> lock(engine_queues().mu);
+    engine_queues().busy.erase(engine);
+}
+// Have `stream` wait for the chunks queued on the device; `any`: whether there are.
+cudaError_t wait_for_engines(int device, cudaStream_t stream, bool* any) {
+    std::lock_guard<std::mutex> lock(engine_queues().mu);
+    *any = false;
+    for (const auto& kv : engine_queues().busy) {
+        if (kv.second.first != device) continue;
+        *any = true;
+        const cudaError_t e = cudaStreamWaitEvent(stream, kv.second.second, 0);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 void free_resident(tb_system* s) {
@@ -151,6 +191,9 @@ int run_resident(tb_system* s, SolveCtl* out) {
     const ResidentKernel kernel = P.mute ? resident_kernel<true>(s->res_nodes, tl) : resident_kernel<false>(s->res_nodes, tl);
     void* args[] = {&P};
     for (long long n = 0;; ++n) {
+        bool shared = false;
+        TB_CUDA(wait_for_engines(s->device, s->stream, &shared));
+        P.limit = shared ? std::min(s->res_params.limit, kResLimitShared) : s->res_params.limit;
         if (cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel),
                                         dim3(s->test_refuse == 2 ? 1 << 16 : s->res_blocks), dim3(kResThreads), args,
                                         s->res_smem, s->stream) != cudaSuccess) {

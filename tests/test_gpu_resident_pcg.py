@@ -285,3 +285,51 @@ def test_two_iterations_match_fp64(ns_local, slabs, rows, cols, fixed, void, smo
     eps = np.finfo(np.float32).eps
     assert np.all(np.abs(got - expected)[free] <= 32 * eps * bound[free])
     assert np.linalg.norm((got - expected)[free]) <= 8 * eps * np.linalg.norm(bound[free])
+
+
+def test_small_solves_leave_a_batch_engine_its_share(ns_local):
+    """A thread of small solves beside a batch: both get on, with the same bits as
+    alone.  The batch took six times as long with launches that did not wait for
+    the engine's; the bound is three."""
+
+    import threading
+    import time
+
+    from pcb_analysis_b200 import serve
+    from pcb_analysis_b200._native import BatchEngine
+
+    requests = [serve.board_request(workloads.board_random(i, side=(150 + 5 * i, 150 + 5 * i), slabs=(8, 8)))
+                for i in range(6)]
+    op = ns_local.MatrixFreeThermalOperator(workloads.board_c1(0, None, 96, 80), preconditioner="two-level")
+    try:
+        with BatchEngine(capacity=6, max_slabs=8, tile_rows=16, preconditioner="two-level") as engine:
+            def batch():
+                start = time.perf_counter()
+                results = serve.solve_batch(requests, CONFIG, engine=engine)
+                return time.perf_counter() - start, results
+
+            rhs = op.build_rhs(op.default_reference_temperature())
+            alone = op.device_system.solve_mpir(rhs, CONFIG)
+            batch()
+            seconds, expected = batch()
+            beside, stop = [], threading.Event()
+
+            def small():
+                while not stop.is_set():
+                    beside.append(op.device_system.solve_mpir(rhs, CONFIG))
+
+            thread = threading.Thread(target=small)
+            thread.start()
+            try:
+                shared_seconds, shared = batch()
+            finally:
+                stop.set()
+                thread.join()
+    finally:
+        op.close()
+    assert beside
+    for result in beside:
+        np.testing.assert_array_equal(result["solution"], alone["solution"])
+    for got, want in zip(shared, expected):
+        np.testing.assert_array_equal(got.solution, want.solution)
+    assert shared_seconds <= 3.0 * seconds
