@@ -83,6 +83,13 @@ struct MLGrid {
 // worse (c3: 559 iterations with 2 x 2 only on grids wider than 200 columns).
 // On a small board the extra levels cost more in launch latency than they
 // save (c2, 3.4 M nodes: 464 -> 452 iterations but 0.056 -> 0.073 s).
+// Those figures are of five kernels per level.  With two, milliseconds and
+// iterations of a solve with 2 x 2 / 4 x 4, by columns across level 1 (seed 1):
+//   c2 rules, 129: 49.0 (439) / 43.7 (453)   c3 rules, 129: 54.8 (419) / 51.2 (441)
+//             176: 56.6 (351) / 71.0 (496)             198: 108 (425) / 128 (577)
+//             198: 97.5 (472) / 96.1 (529)             257: 161 (451) / 197 (576)
+//             226: 114 (468) / 115 (522)               513: 542 (449) / 720 (591)
+// so the line could lie lower, near 150; it stands where it was.
 constexpr int kMlWideSide = 200;
 __host__ __device__ constexpr int ml_aggregate_width(int level, int ny1, int nx1) {  // ny1, nx1: level 1's grid
     return level == 0 ? kMlAgg : ((ny1 > kMlWideSide || nx1 > kMlWideSide) ? 2 : 4);

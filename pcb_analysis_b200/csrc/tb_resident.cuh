@@ -7,11 +7,25 @@
 // the z-march of the operator's few tiles, and after each reduction a ticket,
 // a last block and a scalar read back by the next kernel.  Here one block per
 // SM keeps its share of the nodes, their operator rows and vectors in
-// registers for many iterations.  Measured (12-slab boards of 64 .. 118 cells a
-// side, 55 .. 220 thousand nodes): 12.9 .. 15.9 us an iteration against 31 .. 33
-// with the two-level preconditioner, 7.0 .. 9.0 against 17 .. 19 with Jacobi.
+// registers for many iterations (with two nodes a thread, above 113 thousand
+// padded nodes, some 100 bytes a thread of them spill to local memory).
+// Measured (12-slab boards of 64 .. 118 cells a side, 55 .. 220 thousand nodes):
+// 13.0 .. 16.0 us an iteration against 30 .. 31 with the two-level
+// preconditioner, 6.7 .. 8.7 against 15 .. 19 with Jacobi; 128 x 128 x 8: 16.9
+// against 32, and 8.3 against 18.
 // What is left is the round trips: about 1.5 us for each of the two exchanges
 // and 1 us for each of the words of the direction, the patch sums and c.
+//
+// One launch has the whole device, so solves of several host threads follow one
+// another where the graph-captured kernels overlap.  Milliseconds per solve with
+// 1 / 2 / 3 / 4 / 8 threads, this kernel and the graph-captured ones:
+//   64 x 64 x 8 two-level     19.6 17.1 17.2 16.7 17.3     46.5 24.3 16.9 14.2 10.7
+//   120 x 120 x 8 two-level   49.7 47.8 45.8 43.9 45.0     93.5 55.3 42.9 36.0 33.0
+//   96 x 80 x 8 Jacobi        61.3 60.7 59.9 57.9 59.5     135  81.2 55.2 45.5 33.1
+//   24 x 24 x 8 two-level      4.4  3.5  2.6  2.6  2.3     12.5 10.2  7.2  5.9  4.2
+// Which kernels a solve takes does not depend on what else runs, so that its bits
+// do not; a program with four or more such solves at a time sets a launch plan
+// (tb_set_apply_plan), or hands its boards to a batch engine.
 //
 // What the blocks tell each other travels in 64-bit words that carry their own
 // tag (the iteration) beside the FP32 value, so that no fence or flag has to
@@ -60,7 +74,7 @@
 
 namespace tb {
 
-constexpr int kResThreads = 768;   // 80 registers a thread: two nodes' rows of 27 coefficients
+constexpr int kResThreads = 768;   // 80 registers a thread: most of two nodes' rows of 27 coefficients
 constexpr int kResNodes = 2;       // nodes per thread at most
 constexpr int kResRow = 27;        // s_d (8 columns), a_d- and a_d+ (9 each), and the Robin term
 constexpr int kResMaxBlocks = 160; // blocks whose posts one exchange reads (five warps)
